@@ -78,8 +78,10 @@ _SIGS = {
     "mmj_col2im": ([P, P, P, L, I, P], 1),
     "mmj_conv2d_fwd": ([P, P, P, P, P, I, P], 1),
     "mmj_conv2d_dx": ([P, P, P, P, P, I, P], 1),
-    "mmj_conv2d_dw": ([P, P, P, P, I, P], 1),
-    "mmj_channel_sum": ([P, P, I, I, L, I, P], 1),
+    "mmj_conv2d_dw": ([P, P, P, P, P, I, P], 2),
+    "mmj_conv2d_dw_scratch": ([P], 0),
+    "mmj_channel_sum": ([P, P, P, I, I, L, I, P], 2),
+    "mmj_channel_sum_splits": ([I, I], 0),
     "mmj_maxpool2d_fwd": ([P, P, P, P, I, P], 1),
     "mmj_maxpool2d_bwd": ([P, P, P, P, I, P], 1),
     "mmj_avgpool2d_fwd": ([P, P, P, I, P], 1),
@@ -118,7 +120,8 @@ _SIGS = {
     "mmj_set_signal_slots": ([I], 0),
 }
 
-_OPTIONAL = {}
+# launchers that do not return a status code
+_OPTIONAL = {"mmj_conv2d_dw_scratch": L}
 
 
 DEBUG_BOUNDS = os.environ.get("MOMIJO_DEBUG_BOUNDS", "0") == "1"

@@ -78,6 +78,22 @@ def col2im(cols, x_shape, kernel, stride=(1, 1), pad=(0, 0), dilation=(1, 1)):
 
 
 # ---- convolution ----------------------------------------------------------------------------------------
+def _weight_grad(x, dy, w, geom):
+    dw = torch.empty_like(w)
+    n = _C.lib().mmj_conv2d_dw_scratch(geom)
+    scratch = torch.empty(n, dtype=torch.float32, device=x.device) if n else None
+    _C.call("mmj_conv2d_dw", _C.ptr(x), _C.ptr(dy), _C.ptr(dw), _C.ptr(scratch), geom, _dt(x), _C.current_stream())
+    return dw
+
+
+def _channel_sum(dy, N, C, spatial):
+    """Sums of a [N, C, spatial] tensor over images and positions (bias gradient)."""
+    db = torch.empty(C, dtype=dy.dtype, device=dy.device)
+    scratch = torch.empty(_C.lib().mmj_channel_sum_splits(N, C) * C, dtype=torch.float32, device=dy.device)
+    _C.call("mmj_channel_sum", _C.ptr(dy), _C.ptr(db), _C.ptr(scratch), N, C, spatial, _dt(dy), _C.current_stream())
+    return db
+
+
 def _use_gemm(x, w, groups):
     """bf16 with a contraction of at least 64 and a few thousand output positions: lower to the tensor cores."""
     K = w.shape[1] * w.shape[2] * w.shape[3]
@@ -136,11 +152,9 @@ class _Conv2d(torch.autograd.Function):
                 dx = torch.empty_like(x)
                 _C.call("mmj_conv2d_dx", _C.ptr(dy), _C.ptr(w), None, _C.ptr(dx), ctx.geom, _dt(x), _C.current_stream())
             if ctx.needs_input_grad[1]:
-                dw = torch.empty_like(w)
-                _C.call("mmj_conv2d_dw", _C.ptr(x), _C.ptr(dy), _C.ptr(dw), ctx.geom, _dt(x), _C.current_stream())
+                dw = _weight_grad(x, dy, w, ctx.geom)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = torch.empty(OC, dtype=dy.dtype, device=dy.device)
-            _C.call("mmj_channel_sum", _C.ptr(dy), _C.ptr(db), N, OC, OH * OW, _dt(dy), _C.current_stream())
+            db = _channel_sum(dy, N, OC, OH * OW)
         return dx, dw, db, None, None, None, None
 
 
@@ -187,11 +201,9 @@ class _ConvTranspose2d(torch.autograd.Function):
             dx = torch.empty_like(x)   # the associated convolution's forward applied to dy
             _C.call("mmj_conv2d_fwd", _C.ptr(dy), _C.ptr(w), None, _C.ptr(dx), ctx.geom, _dt(x), _C.current_stream())
         if ctx.needs_input_grad[1]:
-            dw = torch.empty_like(w)   # its weight gradient with (input, output gradient) = (dy, x)
-            _C.call("mmj_conv2d_dw", _C.ptr(dy), _C.ptr(x), _C.ptr(dw), ctx.geom, _dt(x), _C.current_stream())
+            dw = _weight_grad(dy, x, w, ctx.geom)   # its weight gradient with (input, output gradient) = (dy, x)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = torch.empty(Cout, dtype=dy.dtype, device=dy.device)
-            _C.call("mmj_channel_sum", _C.ptr(dy), _C.ptr(db), N, Cout, Hout * Wout, _dt(dy), _C.current_stream())
+            db = _channel_sum(dy, N, Cout, Hout * Wout)
         return dx, dw, db, None, None, None, None
 
 

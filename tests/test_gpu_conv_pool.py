@@ -104,3 +104,30 @@ def test_layers_use_native_kernels():
     y.sum().backward()
     assert _C.launches - before >= 5
     assert conv.weight.grad is not None and y.shape == (2, 8, 8, 8)
+
+
+@pytest.mark.parametrize("N,C,H,W,OC,k,s,p,d,g", [
+    (1, 1, 5, 7, 1, 3, 1, 1, 1, 1),          # one filter, fewer positions than a tile
+    (2, 3, 13, 11, 17, 5, 2, 2, 1, 1),       # a row past a 16-channel tile; strided classes of unequal size
+    (1, 33, 9, 9, 65, 3, 1, 1, 1, 1),        # a channel past a 32- and a 64-channel tile
+    (3, 16, 12, 10, 48, 1, 3, 0, 1, 1),      # stride larger than the kernel: classes that meet no tap
+    (2, 8, 15, 14, 12, 3, 2, 2, 2, 2),       # dilation and stride share a factor; groups
+    (1, 4, 20, 20, 4, 3, 1, 1, 1, 4),        # depthwise stays with the direct kernels
+    (2, 5, 6, 6, 7, (1, 5), (4, 1), (0, 2), (1, 1), 1),
+    (16, 64, 60, 60, 64, 3, 1, 1, 1, 1),     # several slices and full tiles
+])
+def test_conv2d_tile_edges_against_64_bits(N, C, H, W, OC, k, s, p, d, g):
+    kh, kw = (k, k) if isinstance(k, int) else k
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    r = lambda *shape: torch.randn(*shape, generator=gen, device="cuda").requires_grad_()
+    x, w, b = r(N, C, H, W), r(OC, C // g, kh, kw), r(OC)
+    y = cv.conv2d(x, w, b, s, p, d, g)
+    dy = torch.randn_like(y)
+    got = [y, *torch.autograd.grad(y, [x, w, b], dy)]
+    x64, w64, b64 = (v.detach().double().requires_grad_() for v in (x, w, b))
+    y64 = tF.conv2d(x64, w64, b64, s, p, d, g)
+    want = [y64, *torch.autograd.grad(y64, [x64, w64, b64], dy.double())]
+    # rounding of a sum of n products grows like sqrt(n) * 2^-24 of its norm; 4x for the spread of one draw
+    terms = [C // g * kh * kw, OC // g * kh * kw, N * y.shape[2] * y.shape[3], N * y.shape[2] * y.shape[3]]
+    for a, e, n in zip(got, want, terms):
+        assert float((a.double() - e).norm()) <= 4 * 2.0 ** -24 * (n + 1) ** 0.5 * float(e.norm()) + 1e-12
