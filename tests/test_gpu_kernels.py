@@ -337,3 +337,22 @@ def test_dependent_launch_gives_the_same_bits_as_plain_stream_order():
         assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
         res[pdl] = [l for l in r.stdout.splitlines() if l.startswith("CHAIN")][0]
     assert res["1"] == res["0"]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,shift", [(1, 0), (3, 1), (8, 3), (4099, 5), (3_000_001, 1)])
+def test_sq_norm_edges(dtype, n, shift):
+    """Pieces in front of the first 16-byte boundary and behind the last one; each non-finite value is found."""
+    base = torch.randn(n + shift, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda").to(dtype)
+    x = base[shift:]
+    want = float(x.double().square().sum())
+    found = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = float(ops.sq_norm(x, found_inf=found))
+    assert abs(got - want) <= 4 * 2.0 ** -24 * max(1.0, n / 300000) ** 0.5 * 32 * want and int(found) == 0
+    for at in {0, n // 2, n - 1}:
+        for bad in (float("inf"), float("nan")):
+            y = base.clone()[shift:]
+            y[at] = bad
+            found.zero_()
+            ops.sq_norm(y, found_inf=found)
+            assert int(found) == 1
