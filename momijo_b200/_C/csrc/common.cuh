@@ -340,6 +340,15 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
                : "memory");
 }
 
+// The same arrival on the mbarrier at one shared-memory offset in both CTAs of the pair, in one instruction.
+__device__ __forceinline__ void umma_commit_pair_both(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
+
 // 32 lanes x 32 consecutive fp32 columns: thread i of the warp gets lane (base_lane + i).
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -389,6 +398,16 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   d |= (uint64_t)1 << 46;  // descriptor version for sm_100
   d |= (uint64_t)2 << 61;  // SWIZZLE_128B
   return d;
+}
+
+// The same descriptor as (constant upper half, address-dependent lower half): stepping to another k slice or
+// stage is one 32-bit add on the lower half.
+constexpr uint32_t kSmemDescHi1024 = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
+  return ((smem_addr >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
+}
+__device__ __forceinline__ uint64_t smem_desc(uint32_t lo) {
+  return ((uint64_t)kSmemDescHi1024 << 32) | lo;
 }
 
 // Instruction descriptor for kind::f16 with bf16 inputs and fp32 accumulation.

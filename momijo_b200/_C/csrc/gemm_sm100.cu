@@ -708,6 +708,115 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 constexpr int kPairBN = 256;
 constexpr int kPairStageBytes = kAStageBytes + (kPairBN / 2) * kGemmBK * 2;  // 32 KiB
 
+// Two fp32 values in one register pair: the f32x2 instructions take half the issue slots of scalar ones and round
+// alike. The fused GELU / GELU' epilogues are bound by issue (25 and 28 instructions an element at 41 % of the
+// issue slots, two or three warps per scheduler), not by a pipe.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// the two bf16 halves of a word, widened (their bits are the upper halves of the fp32 values)
+__device__ __forceinline__ f32x2 f2_from_bf16(uint32_t u) {
+  return f2_pack(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+__device__ __forceinline__ uint32_t f2_to_bf16(f32x2 v) {
+  float a, b;
+  f2_unpack(v, a, b);
+  return pack_bf16x2(a, b);
+}
+constexpr float kGeluK0 = 0.7978845608028654f, kGeluK1 = 0.7978845608028654f * 0.044715f;
+__device__ __forceinline__ f32x2 f2_tanh(f32x2 u) {
+  float a, b;
+  f2_unpack(u, a, b);
+  return f2_pack(tanh_fast(a), tanh_fast(b));
+}
+__device__ __forceinline__ f32x2 f2_gelu(f32x2 x) {
+  const f32x2 x2 = f2_mul(x, x);
+  const f32x2 t = f2_tanh(f2_mul(x, f2_fma(x2, f2_pack(kGeluK1, kGeluK1), f2_pack(kGeluK0, kGeluK0))));
+  const f32x2 h = f2_mul(x, f2_pack(0.5f, 0.5f));
+  return f2_fma(h, t, h);
+}
+__device__ __forceinline__ f32x2 f2_gelu_grad(f32x2 x) {
+  const f32x2 x2 = f2_mul(x, x), half = f2_pack(0.5f, 0.5f), one = f2_pack(1.f, 1.f);
+  const f32x2 k0 = f2_pack(kGeluK0, kGeluK0);
+  const f32x2 t = f2_tanh(f2_mul(x, f2_fma(x2, f2_pack(kGeluK1, kGeluK1), k0)));
+  const f32x2 du = f2_fma(x2, f2_pack(3.f * kGeluK1, 3.f * kGeluK1), k0);
+  const f32x2 sech2 = f2_fma(f2_mul(t, f2_pack(-1.f, -1.f)), t, one);
+  return f2_fma(f2_mul(f2_mul(x, half), sech2), du, f2_fma(t, half, half));
+}
+
+// Stores 32 rows x 32 bf16 columns (lane = row, 16 packed words) through the warp's staging area.
+__device__ __forceinline__ void staged_store_words(uint8_t* st, int lane, const uint32_t (&w)[16],
+                                                   __nv_bfloat16* tile, long long ld) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<uint4*>(st + stage_off(lane, i)) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int rr = 8 * i + (lane >> 2);
+    const uint4 q = *reinterpret_cast<const uint4*>(st + stage_off(rr, lane & 3));
+    *reinterpret_cast<uint4*>(tile + rr * ld + (lane & 3) * 8) = q;
+  }
+  __syncwarp();
+}
+
+// Epilogue of a full 32-row, 32-column chunk with the options fixed at compile time. kMode: 1 = bf16 result with an
+// optional bias, 2 = bias, pre-activation kept, GELU, 3 = times GELU'(aux). `bias` / `auxq` hold the chunk's 16 words.
+template <int kMode>
+__device__ __forceinline__ void epilogue_chunk_fixed(const GemmParams& p, const uint32_t (&acc)[32], bool has_bias,
+                                                     const uint4 (&extra)[4], long long row0, int col0, uint8_t* st,
+                                                     int lane) {
+  const uint32_t* ew = reinterpret_cast<const uint32_t*>(extra);
+  uint32_t w[16];
+  if (kMode == 2) {
+    uint32_t act[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      f32x2 v = f2_pack(__uint_as_float(acc[2 * i]), __uint_as_float(acc[2 * i + 1]));
+      if (has_bias) v = f2_add(v, f2_from_bf16(ew[i]));
+      w[i] = f2_to_bf16(v);
+      act[i] = f2_to_bf16(f2_gelu(v));
+    }
+    staged_store_words(st, lane, w, reinterpret_cast<__nv_bfloat16*>(p.D2) + row0 * p.ldd2 + col0, p.ldd2);
+    staged_store_words(st, lane, act, reinterpret_cast<__nv_bfloat16*>(p.D) + row0 * p.ldd + col0, p.ldd);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    f32x2 v = f2_pack(__uint_as_float(acc[2 * i]), __uint_as_float(acc[2 * i + 1]));
+    if (kMode == 1) {
+      if (has_bias) v = f2_add(v, f2_from_bf16(ew[i]));
+    } else {
+      v = f2_mul(v, f2_gelu_grad(f2_from_bf16(ew[i])));
+    }
+    w[i] = f2_to_bf16(v);
+  }
+  staged_store_words(st, lane, w, reinterpret_cast<__nv_bfloat16*>(p.D) + row0 * p.ldd + col0, p.ldd);
+}
+
+// kMode 0: every combination of epilogue options; 1 to 3: the fixed ones of epilogue_chunk_fixed.
+template <int kMode>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
@@ -802,18 +911,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       }
     } else if (warp == 1) {
       // ======================= MMA issuer (rank 0 only) =======================
-      if (lane == 0 && leader) {
+      // The whole warp walks the loop and an elected lane issues; stage descriptors are one addition and both CTAs'
+      // barriers take one multicast commit. With lane 0 alone in a divergent loop and two commits, a 64-deep K block
+      // cost about 900 cycles of issue against 512 of tensor time: 16384 x 2304 x 768 51.0 -> 47.2 us,
+      // x 768 x 3072 64.0 -> 57.9, x 50304 x 768 1058 -> 991 (cuBLAS 47.5, 58.0, 1072 beside it). The one-SM kernel
+      // keeps lane 0: its 256-row tiles have twice the tensor time per block, and measured 349 -> 376 us this way.
+      if (leader) {
         const uint32_t idesc = make_idesc_bf16(2 * kGemmBM, kPairBN, p.a_mn, p.b_mn);
         const uint32_t a_lbo = p.a_mn ? 8192u : 16u;
         const uint32_t b_lbo = p.b_mn ? 8192u : 16u;
-        const uint32_t a_kstep = p.a_mn ? 2048u : 32u;
-        const uint32_t b_kstep = p.b_mn ? 2048u : 32u;
-        const uint32_t empty_own = smem_u32(&empty_bar[0]);
-        const uint32_t empty_peer = mapa_shared(empty_own, 1);
-        const uint32_t tfull_own = smem_u32(&tfull_bar[0]);
-        const uint32_t tfull_peer = mapa_shared(tfull_own, 1);
-        const uint32_t empty_own_c = mapa_shared(empty_own, 0);
-        const uint32_t tfull_own_c = mapa_shared(tfull_own, 0);
+        const uint32_t a_kstep = (p.a_mn ? 2048u : 32u) >> 4;
+        const uint32_t b_kstep = (p.b_mn ? 2048u : 32u) >> 4;
+        const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), a_lbo);
+        const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem) + (uint32_t)kAStageBytes, b_lbo);
         int s = 0;
         uint32_t ph = 0;
         int acc = 0;
@@ -822,34 +932,29 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         for (int t = pair; t < num_tiles && ok; t += num_pairs) {
           const KRange kr = krange_of(t, per_group, num_k, p);
           if (kr.nk == 0) continue;  // empty contraction: the epilogues write zeros on their own
-          if (!mbar_wait(&tempty_bar[acc], acc_ph ^ 1, &abort_flag, p.status, kTimeoutTmemEmpty,
-                         t)) {
-            break;
-          }
+          if (!mbar_wait_warp(&tempty_bar[acc], acc_ph ^ 1, &abort_flag, p.status, kTimeoutTmemEmpty, t)) break;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(acc * kAccCols);
           for (int kb = 0; kb < kr.nk; ++kb) {
-            if (!mbar_wait(&full_bar[s], ph, &abort_flag, p.status, kTimeoutFull, kb)) {
+            if (!mbar_wait_warp(&full_bar[s], ph, &abort_flag, p.status, kTimeoutFull, kb)) {
               ok = false;
               break;
             }
             tc_fence_after();
-            const uint32_t a_base = smem_u32(smem + (size_t)s * kPairStageBytes);
-            const uint32_t b_base = a_base + (uint32_t)kAStageBytes;
+            if (elect_one()) {
+              const uint32_t a_lo = a_lo0 + (uint32_t)(s * (kPairStageBytes >> 4));
+              const uint32_t b_lo = b_lo0 + (uint32_t)(s * (kPairStageBytes >> 4));
 #pragma unroll
-            for (int k = 0; k < kGemmBK / 16; ++k) {
-              const uint64_t da = make_smem_desc(a_base + k * a_kstep, a_lbo, 1024);
-              const uint64_t db = make_smem_desc(b_base + k * b_kstep, b_lbo, 1024);
-              umma_bf16_ss_pair(d_tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < kGemmBK / 16; ++k)
+                umma_bf16_ss_pair(d_tmem, smem_desc(a_lo + k * a_kstep), smem_desc(b_lo + k * b_kstep), idesc,
+                                  (kb > 0 || k > 0) ? 1u : 0u);
+              // the stage is free in both CTAs once these MMAs retire
+              umma_commit_pair_both(&empty_bar[s]);
+              if (kb + 1 == kr.nk) umma_commit_pair_both(&tfull_bar[acc]);
             }
-            // the stage is free in both CTAs once these MMAs retire
-            umma_commit_pair(empty_own_c + (uint32_t)(s * sizeof(uint64_t)));
-            umma_commit_pair(empty_peer + (uint32_t)(s * sizeof(uint64_t)));
+            __syncwarp();
             if (++s == stages) { s = 0; ph ^= 1; }
           }
-          if (!ok) break;
-          umma_commit_pair(tfull_own_c + (uint32_t)(acc * sizeof(uint64_t)));
-          umma_commit_pair(tfull_peer + (uint32_t)(acc * sizeof(uint64_t)));
           if (++acc == 2) { acc = 0; acc_ph ^= 1; }
         }
       }
@@ -889,6 +994,43 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         const int row = m0 + quad * 32 + lane;
         const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * kAccCols);
         uint8_t* st = (m0 + quad * 32 + 32 <= p.M) ? epi_stage[warp - 2] : nullptr;
+        if (kMode != 0 && st != nullptr && n0 + kPairBN <= p.N) {
+          // full tile: the next chunk's accumulator and operand are requested before this chunk is worked on
+          const bool has_bias = kMode != 3 && (p.epi & kEpiBias) != 0;
+          const uint4* ext = kMode == 3
+              ? reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.aux) + (long long)row * p.ldaux + n0)
+              : reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.bias) + n0);
+          const long long row0 = m0 + quad * 32;
+          uint32_t r[2][32];
+          uint4 e[2][4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) e[0][i] = e[1][i] = make_uint4(0u, 0u, 0u, 0u);
+          tmem_ld_32x32(t_row + (uint32_t)(chalf * 32), r[0]);
+          if (kMode == 3 || has_bias) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) e[0][i] = __ldg(ext + chalf * 4 + i);
+          }
+#pragma unroll
+          for (int j = 0; j < kPairBN / 64; ++j) {
+            const int c = chalf + 2 * j;
+            tmem_ld_wait();
+            if (j + 1 < kPairBN / 64) {
+              tmem_ld_32x32(t_row + (uint32_t)((c + 2) * 32), r[(j + 1) & 1]);
+              if (kMode == 3 || has_bias) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) e[(j + 1) & 1][i] = __ldg(ext + (c + 2) * 4 + i);
+              }
+            } else {
+              // every column is in registers: the accumulator can be overwritten while they are worked on
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(tempty0 + (uint32_t)(acc * sizeof(uint64_t)));
+            }
+            epilogue_chunk_fixed<kMode>(p, r[j & 1], has_bias, e[j & 1], row0, n0 + c * 32, st, lane);
+          }
+          if (++acc == 2) { acc = 0; acc_ph ^= 1; }
+          continue;
+        }
         // The aux operand of the GELU' / add / multiply epilogues is requested one chunk ahead, so that
         // its latency hides behind the previous chunk instead of following every TMEM read.
         const bool has_aux = (p.epi & (kEpiDGelu | kEpiAddAux | kEpiMulAux)) != 0 && p.vec_ok && row < p.M;
@@ -1151,11 +1293,15 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
   const int smem_bytes = stages * kPairStageBytes + 1024;
   if (g_pair_max_dyn == 0) {
     cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, gemm_bf16_pair_kernel);
+    typedef void (*PairKernel)(CUtensorMap, CUtensorMap, GemmParams);
+    cudaError_t e = cudaFuncGetAttributes(&fa, gemm_bf16_pair_kernel<0>);
     if (e != cudaSuccess) return (int)e;
     const int max_dyn = 232448 - (int)fa.sharedSizeBytes;
-    e = cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
-    if (e != cudaSuccess) return (int)e;
+    for (PairKernel k : {&gemm_bf16_pair_kernel<0>, &gemm_bf16_pair_kernel<1>, &gemm_bf16_pair_kernel<2>,
+                         &gemm_bf16_pair_kernel<3>}) {
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
+      if (e != cudaSuccess) return (int)e;
+    }
     // how many pairs the device holds at once (a persistent grid must not exceed it)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * sm_count());
@@ -1167,7 +1313,7 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<0>, &cfg);
     if (e != cudaSuccess || n <= 0) { cudaGetLastError(); n = sm_count() / 2; }
     g_pair_clusters = n;
     g_pair_max_dyn = max_dyn;
@@ -1181,8 +1327,14 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
   if (tiles < pairs) pairs = (int)tiles;
   p.gemm_ctas = 2 * pairs;
   {
-    cudaError_t e = launch_pdl(gemm_bf16_pair_kernel, dim3(2 * pairs), dim3(kThreads), (size_t)smem_bytes, stream,
-                               tmA, tmB, p);
+    // the epilogues of the main path are compiled on their own (vector access throughout, ordinary output)
+    auto* kernel = &gemm_bf16_pair_kernel<0>;
+    if (p.vec_ok && p.groups_k == 0) {
+      if ((p.epi & ~kEpiBias) == 0) kernel = &gemm_bf16_pair_kernel<1>;
+      else if ((p.epi & ~kEpiBias) == kEpiGelu) kernel = &gemm_bf16_pair_kernel<2>;
+      else if (p.epi == kEpiDGelu) kernel = &gemm_bf16_pair_kernel<3>;
+    }
+    cudaError_t e = launch_pdl(kernel, dim3(2 * pairs), dim3(kThreads), (size_t)smem_bytes, stream, tmA, tmB, p);
     if (e != cudaSuccess) return (int)e;
   }
   return (int)cudaGetLastError();

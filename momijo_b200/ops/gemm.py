@@ -117,6 +117,16 @@ def pick_tall(M: int, N: int, K: int) -> bool:
     return K >= 4096 and M >= 256 and N >= 256 and (-(-M // 256)) * (-(-N // 256)) >= 3 * 148
 
 
+def tall_beats_pair(M: int, N: int, K: int) -> bool:
+    """One-SM 256 x 256 tiles instead of CTA pairs: products with a very long contraction, unless whole-SM tiles
+    leave a longer last wave. Measured, tall / pair, us: 4096 x 4096 x 28672 631 / 679, 16384 x 4096 x 8192 716 / 774,
+    50304 x 768 x 16384 818 / 870; at K = 4096 the order turns (4096 x 28672 638 / 592, 4096 x 14336 331 / 314)."""
+    if K < 8192:
+        return False
+    tiles = -(-M // 256) * -(-N // 256)
+    return 2 * -(-tiles // 148) <= -(-tiles // 74)
+
+
 def pick_pair(M: int, N: int, K: int) -> bool:
     """CTA-pair kernel for plain products: each SM of a pair stages half of the 256-wide B tile, so a
     256 x 256 tile costs a third less L2 -> shared-memory traffic per FLOP than 128 x 256 on one SM, and
@@ -126,9 +136,7 @@ def pick_pair(M: int, N: int, K: int) -> bool:
         return False
     if mode == "1":
         return True
-    # measured: ahead of the one-SM tiles by 1.2x on contractions up to 3072 deep (0.88-0.95 of cuBLAS);
-    # long contractions with many tiles stay on the one-SM 256 x 256 tiles (pick_tall)
-    return not pick_tall(M, N, K)
+    return not tall_beats_pair(M, N, K)
 
 
 def _split_ranges(K: int, S: int, device):
@@ -248,7 +256,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_f32=False, accumulate=Fa
     if pair:
         bn, tall = 256 | PAIR, False
     elif bn is None:
-        if not tall and pick_tall(M, N, K):
+        if not tall and M >= 256 and N >= 256 and (pick_tall(M, N, K) or tall_beats_pair(M, N, K)):
             bn, tall = 256, True
         else:
             bn = pick_bn(M, N)
