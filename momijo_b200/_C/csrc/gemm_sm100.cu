@@ -781,7 +781,9 @@ __device__ __forceinline__ void staged_store_words(uint8_t* st, int lane, const 
   __syncwarp();
 }
 
-// Epilogue of a full 32-row, 32-column chunk with the options fixed at compile time. kMode: 1 = bf16 result with an
+// Epilogue of a full 32-row, 32-column chunk (16384 x 3072 x 768: GELU 86 -> 75 us, GELU' 99 -> 78 us, of which 13 us
+// came from fetching aux four lanes to a row instead of a row per lane; sixteen epilogue warps instead of eight measured
+// 78 and 81) with the options fixed at compile time. kMode: 1 = bf16 result with an
 // optional bias, 2 = bias, pre-activation kept, GELU, 3 = times GELU'(aux). `bias` / `auxq` hold the chunk's 16 words.
 template <int kMode>
 __device__ __forceinline__ void epilogue_chunk_fixed(const GemmParams& p, const uint32_t (&acc)[32], bool has_bias,
@@ -977,7 +979,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
             uint32_t z[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) z[i] = 0u;
-            for (int c = chalf; c < kPairBN / 32; c += 2) {
+            for (int c = chalf; c < kPairBN / 32; c += kEpiWarps / 4) {
               const int col0 = n0 + c * 32;
               if (col0 < p.N) {
                 if (p.epi & kEpiOutF32)
@@ -998,35 +1000,52 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
           // full tile: the next chunk's accumulator and operand are requested before this chunk is worked on
           const bool has_bias = kMode != 3 && (p.epi & kEpiBias) != 0;
           const uint4* ext = kMode == 3
-              ? reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.aux) + (long long)row * p.ldaux + n0)
+              ? reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.aux) +
+                                               (long long)(m0 + quad * 32 + (lane >> 2)) * p.ldaux + n0) + (lane & 3)
               : reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.bias) + n0);
           const long long row0 = m0 + quad * 32;
+          constexpr int kStep = kEpiWarps / 4, kChunks = kPairBN / 32 / kStep;
           uint32_t r[2][32];
           uint4 e[2][4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) e[0][i] = e[1][i] = make_uint4(0u, 0u, 0u, 0u);
+          // a bias chunk is the same for every lane; four lanes fetch the 64 bytes of an aux row, eight rows at a time
+          auto fetch = [&](int c, uint4 (&q)[4]) {
+            if (kMode == 3) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                q[i] = __ldg(ext + (long long)(8 * i) * (p.ldaux >> 3) + c * 4);
+            } else if (has_bias) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) q[i] = __ldg(ext + c * 4 + i);
+            }
+          };
           tmem_ld_32x32(t_row + (uint32_t)(chalf * 32), r[0]);
-          if (kMode == 3 || has_bias) {
+          fetch(chalf, e[0]);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) e[0][i] = __ldg(ext + chalf * 4 + i);
-          }
+          for (int j = 0; j < kChunks; ++j) {
+            const int c = chalf + kStep * j;
+            uint4(&q)[4] = e[j & 1];
+            if (kMode == 3) {   // to one row per lane
 #pragma unroll
-          for (int j = 0; j < kPairBN / 64; ++j) {
-            const int c = chalf + 2 * j;
+              for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<uint4*>(st + stage_off(8 * i + (lane >> 2), lane & 3)) = q[i];
+              __syncwarp();
+#pragma unroll
+              for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const uint4*>(st + stage_off(lane, i));
+              __syncwarp();
+            }
             tmem_ld_wait();
-            if (j + 1 < kPairBN / 64) {
-              tmem_ld_32x32(t_row + (uint32_t)((c + 2) * 32), r[(j + 1) & 1]);
-              if (kMode == 3 || has_bias) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) e[(j + 1) & 1][i] = __ldg(ext + (c + 2) * 4 + i);
-              }
+            if (j + 1 < kChunks) {
+              tmem_ld_32x32(t_row + (uint32_t)((c + kStep) * 32), r[(j + 1) & 1]);
+              fetch(c + kStep, e[(j + 1) & 1]);
             } else {
               // every column is in registers: the accumulator can be overwritten while they are worked on
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive_cluster(tempty0 + (uint32_t)(acc * sizeof(uint64_t)));
             }
-            epilogue_chunk_fixed<kMode>(p, r[j & 1], has_bias, e[j & 1], row0, n0 + c * 32, st, lane);
+            epilogue_chunk_fixed<kMode>(p, r[j & 1], has_bias, q, row0, n0 + c * 32, st, lane);
           }
           if (++acc == 2) { acc = 0; acc_ph ^= 1; }
           continue;
@@ -1046,15 +1065,15 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
             aq_next[i] = reinterpret_cast<const uint4*>(aux_row + n0 + chalf * 32)[i];
           aq_next_ok = true;
         }
-        for (int c = chalf; c < kPairBN / 32; c += 2) {
+        for (int c = chalf; c < kPairBN / 32; c += kEpiWarps / 4) {
           uint32_t r[32];
           tmem_ld_32x32(t_row + (uint32_t)(c * 32), r);
 #pragma unroll
           for (int i = 0; i < 4; ++i) aq[i] = aq_next[i];
           aq_ok = aq_next_ok;
           aq_next_ok = false;
-          const int ncol0 = n0 + (c + 2) * 32;
-          if (has_aux && c + 2 < kPairBN / 32 && ncol0 + 32 <= p.N) {
+          const int ncol0 = n0 + (c + kEpiWarps / 4) * 32;
+          if (has_aux && c + kEpiWarps / 4 < kPairBN / 32 && ncol0 + 32 <= p.N) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) aq_next[i] = reinterpret_cast<const uint4*>(aux_row + ncol0)[i];
             aq_next_ok = true;
