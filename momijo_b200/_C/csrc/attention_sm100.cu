@@ -6,11 +6,11 @@
 //   S = Q K^T in TMEM -> softmax warps read one row per thread (no shuffles needed), keep the
 //   running max / sum, write P (bf16) into shared memory in the swizzled K-major layout ->
 //   O_part = P V in TMEM -> threads fold O_part into a register accumulator.
-// Backward, one CTA per (128 key rows, kv head, batch), looping over the query blocks (and,
+// Backward, per item of 128 key rows of one (kv head, batch), looping over the query blocks (and,
 // for GQA, over the query heads of the group):
 //   S^T = K Q^T and dP^T = V dO^T (TMEM) -> threads rebuild P^T = exp(S^T*scale - lse) and
-//   dS^T = P^T o (dP^T - delta), write both to shared memory -> dV += P^T dO, dK += dS^T Q
-//   (TMEM, accumulated over the whole loop), dQ = dS K (TMEM, then a TMA reduce-add into the
+//   dS^T = P^T o (dP^T - delta) and write both back to tensor memory -> dV += P^T dO, dK += dS^T Q
+//   (TMEM, accumulated over the whole loop), dQ^T = K^T dS^T (TMEM, then a TMA reduce-add into the
 //   fp32 accumulator in global memory).
 // The tiles loaded once by TMA serve both as K-major and as MN-major operands: a 128-row tile
 // whose rows are 128 swizzled bytes is the canonical layout of either, read with a different
@@ -25,9 +25,6 @@
 namespace mmj {
 
 constexpr int kAttnThreads = 192;     // forward: TMA warp, MMA warp, 4 softmax warps
-constexpr int kAttnBwdThreads = 448;  // backward: TMA warp, MMA warp, 8 compute warps, 4 dQ warps
-struct TrueTag { static constexpr bool value = true; };
-struct FalseTag { static constexpr bool value = false; };
 constexpr int kPanelBytes = 128 * 128;  // 128 rows x 64 bf16
 
 struct AttnParams {
@@ -100,7 +97,7 @@ __device__ __forceinline__ void bulk_wait_group0() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// Optional kernel timeline: when a trace buffer is installed, one compute (or softmax) thread and the
+// Optional timeline of the forward kernels: when a trace buffer is installed, one softmax thread and the
 // MMA thread of every CTA store clock64() stamps at their stage boundaries (64 slots per CTA).
 constexpr int kTraceSlots = 64;
 __device__ __forceinline__ void trace_stamp(long long* trace, int cta, int slot) {
@@ -828,118 +825,144 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ O, long long
   }
 }
 
+// Backward kernel: one persistent CTA per SM walks (key block, kv head, batch) items; inside an item it visits
+// 64-query blocks of every query head of the group. Warps: 0 = TMA producer, 1 = issuer of the score products and owner
+// of TMEM, 2 = issuer of the gradient products, 3 = idle, then one (head_dim 128) or two (64) compute groups of eight
+// warps, then four dQ drain warps.
+//
+// What bounds it: a block's chain - scores 1060 cycles, TMEM read / exponential / store 1430, gradients 1230, measured
+// with clock stamps at head_dim 64 - is twice as long as the tensor core's own time (about 55 cycles for each of 24 or 32
+// products, which read 2 to 4 KB of A and B from shared memory each), so blocks have to overlap; at head_dim 128 the
+// L2's rate of fp32 reductions costs another sixth (785 -> 655 us without them).
+//   * 64 queries to a block, because two 128-query blocks do not fit (at head_dim 128 one block of 128 left a single
+//     Q / dO stage, and every block waited out a TMA round trip). Three blocks are in flight at head_dim 64, where two
+//     compute groups take them in turn (two blocks and one group: 160 us against 151; sixteen warps on one block: 170);
+//     tensor memory holds two at head_dim 128, where a second group only lengthens the chain (883 us against 765).
+//   * P^T and dS^T are written back over their scores in tensor memory and are the A operands of dV and dK from there;
+//     dS^T goes to shared memory as well, as the B operand of dQ^T.
+//   * dQ is computed transposed (dQ^T = K^T dS^T, 128 lanes = head_dim, 64 columns = queries) into the columns of the
+//     dP^T it came from. At head_dim 64 the upper 64 lanes read the V tile that lies behind K and are ignored. A drain
+//     warp owns 32 of head_dim and writes rows of 32 contiguous values, conflict free, for a TMA reduce-add (one
+//     red.global per value instead: 2.5 times slower).
+//   * items are dealt in a snake over CTAs, longest first; at head_dim 64 K and V are double-buffered, so that the
+//     next item's scores run under the last block of this one.
+// Measured with the delta kernel, 128-query blocks before -> now, us: B16 T1024 H12 D64 causal 221 -> 151, B4 T4096 H16
+// D64 causal 733 -> 545, B2 T4096 H32:8 D128 causal 1224 -> 765, B6 T1777 H16 D128 full 788 -> 538, B2 T777 H8:2 D128
+// causal 147 -> 73.
+// TMEM columns: buffer b at 128 b: S^T / (P^T, dS^T) 64 | dP^T / dQ^T 64; dV and dK behind the last buffer.
+template <int kWarps>
 struct BwdCtl {
-  uint64_t kv_full, s_full, p_full, pds_free, acc_full, stat_full;
-  uint64_t dq_full[2], dq_read[2];
-  uint64_t dq_staged, stage_free;
-  uint64_t qdo_full[4], qdo_empty[4];
-  float s_lse[2][128], s_delta[2][128];
+  float neg_lse[kWarps][32], neg_delta[kWarps][32];   // one row per compute warp: the 32 query columns it works on
+  uint64_t kv_full[2], kv_empty[2], qdo_full[4], qdo_empty[4];
+  uint64_t s_full[3], pds_full[3], dq_full[3], dq_read[3], ds_free[3], acc_full, acc_empty;
   uint32_t tmem_slot;
   int abort_flag;
 };
 
-// Backward kernel. Warp roles (14 warps): 0 = TMA producer, 1 = MMA issuer and TMEM owner,
-// 2..9 = compute (P^T and dS^T from S^T and dP^T, then the dK/dV epilogue), 10..13 = dQ drain
-// (TMEM -> registers -> swizzled fp32 staging tile -> TMA reduce-add into global; per-thread
-// red.global.add would spend one L1 sector slot per 16 bytes and starve the compute warps' own
-// shared-memory traffic). A warp reaches the 32 TMEM lanes of its quadrant (warp
-// index mod 4) only, so two compute warps share each quadrant and split the columns; two
-// compute warps per scheduler also hide each other's dependent-issue and TMEM-load latency.
+__device__ __forceinline__ void bulk_wait_group_read1() {
+  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+}
+// 16 consecutive 32-bit columns of this thread's lane
+__device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st_32x32(taddr, r); }
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32(taddr, r); }
+
 template <int D>
-__global__ void __launch_bounds__(kAttnBwdThreads, 1)
+struct BwdCfg {
+  static constexpr int kBufs = (D == 64) ? 3 : 2;     // S^T / dP^T buffers (128 TMEM columns each) and dS^T tiles
+  static constexpr int kGroups = (D == 64) ? 2 : 1;   // compute groups of 8 warps; they take the blocks in turn
+  static constexpr int kCols = (D == 64) ? 16 : 32;   // query columns a thread holds at a time (80 / 128 registers)
+  static constexpr int kThreads = (8 + 8 * kGroups) * 32;
+};
+
+template <int D>
+__global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const __grid_constant__ CUtensorMap tmdQ, const AttnParams p) {
   constexpr int NP = D / 64;
-  constexpr int kTile = NP * kPanelBytes;
-  // head_dim 64: three Q/dO stages, so that a stage released by the MMAs of block i is refilled
-  // (about 1.5 us of TMA latency) before block i+2 needs it, and two dQ accumulators.
-  // head_dim 128 has shared memory for one stage and TMEM columns for one dQ that aliases S^T.
-  constexpr int kStages = (D == 64) ? 3 : 1;
-  constexpr bool kAliasdQ = (D == 128);
-  constexpr int kDQB = kAliasdQ ? 1 : 2;
-  constexpr uint32_t kTmemCols = 512;
-  constexpr uint32_t kColSt = 0, kColdPt = 128, kColdV = 256, kColdK = 256 + D;
-  constexpr uint32_t kColdQ = kAliasdQ ? 0u : (256u + 2u * D);  // + D per extra buffer
-  constexpr int kPdsBytes = 2 * kPanelBytes;                    // one 128 x 128 bf16 tile
+  constexpr int kTile = NP * kPanelBytes;      // 128 key rows
+  constexpr int kQPanel = 64 * 128;            // 64 query rows x 64 bf16
+  constexpr int kQTile = NP * kQPanel;         // 64 query rows
+  constexpr int kStages = (D == 64) ? 4 : 3;   // Q / dO blocks in flight
+  constexpr int kKV = (D == 64) ? 2 : 1;       // K / V tiles
+  constexpr int kDrain = D / 32;               // active drain warps
+  constexpr int kDsBytes = 128 * 128;          // 128 keys x 64 queries
+  constexpr int kDqBytes = 32 * 32 * 4;        // 32 queries x 32 of head_dim
+  constexpr int kBufs = BwdCfg<D>::kBufs, kGroups = BwdCfg<D>::kGroups, kCols = BwdCfg<D>::kCols;
+  constexpr uint32_t kTmemCols = 512, kColV = 128 * kBufs, kColK = kColV + D;
 
   extern __shared__ uint8_t smem_raw[];
   // (offset arithmetic on the __shared__ symbol, not an integer round trip, so that the compiler
   // keeps the shared address space and emits shared rather than generic loads and stores)
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint8_t* sK = smem;
-  uint8_t* sV = sK + kTile;
-  uint8_t* sQ = sV + kTile;              // kStages
-  uint8_t* sdO = sQ + kStages * kTile;   // kStages
-  uint8_t* sPt = sdO + kStages * kTile;  // 128 x 128 bf16
-  uint8_t* sdSt = sPt + kPdsBytes;       // 128 x 128 bf16
-  uint8_t* sDQ = sdSt + kPdsBytes;       // 128 x 64 fp32: two 32-column panels, 128-byte swizzle
-
-  // Barriers and the lse / delta staging live behind the tiles in dynamic shared memory: with
-  // head_dim 64 the tiles alone take 224 KB, and a static segment in front of them would push
-  // the 1024-byte alignment padding over the per-CTA limit.
-  BwdCtl& ctl = *reinterpret_cast<BwdCtl*>(sDQ + 2 * kPanelBytes);
+  uint8_t* sKV = smem;                          // kKV x (K | V)
+  uint8_t* sQO = sKV + kKV * 2 * kTile;         // kStages x (Q | dO)
+  uint8_t* sdS = sQO + kStages * 2 * kQTile;    // 2 x dS^T
+  uint8_t* sDQ = sdS + kBufs * kDsBytes;            // 4 warps x 2
+  typedef BwdCtl<8 * kGroups> Ctl;
+  Ctl& ctl = *reinterpret_cast<Ctl*>(sDQ + 8 * kDqBytes);
   {
     uint32_t dyn_bytes;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
-    const uint32_t need = (uint32_t)(reinterpret_cast<uint8_t*>(&ctl) - smem_raw) + sizeof(BwdCtl);
+    const uint32_t need = (uint32_t)(reinterpret_cast<uint8_t*>(&ctl) - smem_raw) + sizeof(Ctl);
     if (need > dyn_bytes) {  // uniform over the CTA: nothing allocated yet, just leave
       if (threadIdx.x == 0) report(p.status, kBadArgument, (int)need);
       return;
     }
   }
-  uint64_t &kv_full = ctl.kv_full, &s_full = ctl.s_full, &p_full = ctl.p_full;
-  uint64_t &pds_free = ctl.pds_free, &acc_full = ctl.acc_full, &stat_full = ctl.stat_full;
-  uint64_t *dq_full = ctl.dq_full, *dq_read = ctl.dq_read;
-  uint64_t &dq_staged = ctl.dq_staged, &stage_free = ctl.stage_free;
-  uint64_t *qdo_full = ctl.qdo_full, *qdo_empty = ctl.qdo_empty;
-  float(*s_lse)[128] = ctl.s_lse;
-  float(*s_delta)[128] = ctl.s_delta;
-  uint32_t& tmem_slot = ctl.tmem_slot;
   int& abort_flag = ctl.abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // One-dimensional grid ordered by work: with a causal mask key block 0 meets every query block and
-  // the last key block only one, so all CTAs of key block 0 are dispatched first, then those of key
-  // block 1 and so on (longest first; the tail of the grid is made of the one-block CTAs).
   const int n_heads_b = p.Hkv * p.B;
-  const int jb = (int)blockIdx.x / n_heads_b;  // key block
-  const int hb = (int)blockIdx.x - jb * n_heads_b;
-  const int hkv = hb % p.Hkv, b = hb / p.Hkv;
   const int group = p.Hq / p.Hkv;
-  const int num_qb = (p.T + 127) / 128;
-  const int kv0 = jb * 128;
-  const int i_begin = p.causal ? jb : 0;
-  const int n_i = num_qb - i_begin;   // query blocks per head
-  const int n_iter = n_i * group;     // (query head in group) x (query block)
-  const int cta_lin = (int)blockIdx.x;
-  const bool tracer = (threadIdx.x == 64);
-  if (tracer) {
-    trace_stamp(p.trace, cta_lin, 0);
-    if (p.trace) {
-      uint32_t smid;
-      asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-      p.trace[(long long)cta_lin * kTraceSlots + 1] = smid;
-      p.trace[(long long)cta_lin * kTraceSlots + 7] = n_iter;
-    }
-  }
+  const int num_qb = (p.T + 63) / 64;
+  const int n_items = ((p.T + 127) / 128) * n_heads_b;
+  const int G = (int)gridDim.x, cta = (int)blockIdx.x;
+  const int rounds = (n_items + G - 1) / G;
+  // item of round k, or -1 (only in the last round). Items are ordered by work: with a causal mask key block 0 meets
+  // every query block and the last key block only its own.
+  auto item_at = [&](int k) -> int {
+    const int w = k * G + ((k & 1) ? G - 1 - cta : cta);
+    return (k < rounds && w < n_items) ? w : -1;
+  };
+  auto first_block = [&](int w) -> int { return p.causal ? 2 * (w / n_heads_b) : 0; };
 
   if (threadIdx.x == 0) {
-    mbar_init(&kv_full, 1);
-    mbar_init(&s_full, 1);
-    mbar_init(&p_full, 8);
-    mbar_init(&pds_free, 1);
-    mbar_init(&acc_full, 1);
-    mbar_init(&stat_full, 128);
-    mbar_init(&dq_staged, 4);
-    mbar_init(&stage_free, 1);
+    mbar_init(&ctl.acc_full, 1);
+    mbar_init(&ctl.acc_empty, kBufs == 3 ? 4 : 8 * kGroups);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&dq_full[s], 1);
-      mbar_init(&dq_read[s], 4);
+      mbar_init(&ctl.kv_full[s], 1);
+      mbar_init(&ctl.kv_empty[s], 1);
+    }
+    for (int s = 0; s < 3; ++s) {
+      mbar_init(&ctl.s_full[s], 1);
+      mbar_init(&ctl.pds_full[s], 8);
+      mbar_init(&ctl.dq_full[s], 1);
+      mbar_init(&ctl.dq_read[s], kDrain);
+      mbar_init(&ctl.ds_free[s], 1);
     }
     for (int s = 0; s < 4; ++s) {
-      mbar_init(&qdo_full[s], 1);
-      mbar_init(&qdo_empty[s], 1);
+      mbar_init(&ctl.qdo_full[s], 1);
+      mbar_init(&ctl.qdo_empty[s], 1);
     }
     abort_flag = 0;
     mbar_fence_init();
@@ -950,343 +973,395 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     prefetch_tmap(&tmdQ);
   }
   if (warp == 1) {
-    tmem_alloc(&tmem_slot, kTmemCols);
+    tmem_alloc(&ctl.tmem_slot, kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_slot;
+  constexpr uint32_t tmem_base = 0;   // an allocation of all 512 columns starts at column 0
   pdl_wait();  // the set-up above read no tensor of the step
   pdl_trigger();
-  if (tracer) trace_stamp(p.trace, cta_lin, 2);
+
+  // dV / dK of item n: 32 key rows (one per lane), 32-column chunks [c0, c1) of head_dim. With one accumulator the
+  // compute warps do this; with two the drain warps do, while the compute warps are already at the next item.
+  // `st`: 2 KB of the calling warp's own, through which rows leave four lanes to 64 bytes; nullptr: a lane stores its
+  // own row.
+  auto store_grads = [&](int quad, int c0, int c1, uint32_t n, int jb, int hkv, int b, uint8_t* st) -> bool {
+    if (!mbar_wait_warp(&ctl.acc_full, n & 1, &abort_flag, p.status, kTimeoutTmemFull, 700)) return false;
+    tc_fence_after();
+    const int row0 = jb * 128 + quad * 32;
+    const uint32_t colV = ((uint32_t)(quad * 32) << 16) + kColV;
+    __nv_bfloat16* dk = p.dK + ((long long)b * p.T + row0) * p.ld_dk + p.dk_col0 + hkv * D;
+    __nv_bfloat16* dv = p.dV + ((long long)b * p.T + row0) * p.ld_dv + p.dv_col0 + hkv * D;
+#pragma unroll 1
+    for (int cc = 2 * c0; cc < 2 * c1; ++cc) {   // dV chunk, dK chunk, ...
+      const bool is_k = cc & 1;
+      const int c = (cc >> 1) * 32;
+      uint32_t r[32];
+      tmem_ld_32x32(colV + (is_k ? D : 0) + c, r);
+      tmem_ld_wait();
+      if (cc + 1 == 2 * c1) {   // in registers: the accumulator may be overwritten
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl.acc_empty);
+      }
+      const float f = is_k ? p.scale : 1.f;
+      __nv_bfloat16* dst = (is_k ? dk : dv) + c;
+      const long long ld = is_k ? p.ld_dk : p.ld_dv;
+      uint4 q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        q[i].x = pack_bf16x2(__uint_as_float(r[8 * i + 0]) * f, __uint_as_float(r[8 * i + 1]) * f);
+        q[i].y = pack_bf16x2(__uint_as_float(r[8 * i + 2]) * f, __uint_as_float(r[8 * i + 3]) * f);
+        q[i].z = pack_bf16x2(__uint_as_float(r[8 * i + 4]) * f, __uint_as_float(r[8 * i + 5]) * f);
+        q[i].w = pack_bf16x2(__uint_as_float(r[8 * i + 6]) * f, __uint_as_float(r[8 * i + 7]) * f);
+      }
+      if (st != nullptr) {
+        // 16-byte pieces of a 64-byte row are XORed with bits 1-2 of the row: conflict free both ways
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(st + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = q[i];
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int rr = 8 * i + (lane >> 2);
+          const uint4 v = *reinterpret_cast<const uint4*>(st + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
+          if (row0 + rr < p.T) reinterpret_cast<uint4*>(dst + rr * ld)[lane & 3] = v;
+        }
+        __syncwarp();
+      } else if (row0 + lane < p.T) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(dst + lane * ld)[i] = q[i];
+      }
+    }
+    return true;
+  };
 
   if (warp == 0) {
+    // ======================= TMA producer =======================
     if (lane == 0) {
-      mbar_expect_tx(&kv_full, 2 * kTile);
+      uint32_t g = 0, n = 0;
+      bool ok = true;
+      for (int k = 0; k < rounds && ok; ++k) {
+        const int w = item_at(k);
+        if (w < 0) break;
+        const int jb = w / n_heads_b, hb = w - jb * n_heads_b;
+        const int hkv = hb % p.Hkv, b = hb / p.Hkv;
+        const int i0 = first_block(w);
+        bool kv_loaded = false;
+        for (int hq = hkv * group; hq < (hkv + 1) * group && ok; ++hq) {
+          for (int qi = i0; qi < num_qb; ++qi, ++g) {
+            const uint32_t s = g % kStages;
+            if (!mbar_wait(&ctl.qdo_empty[s], ((g / kStages) & 1) ^ 1, &abort_flag, p.status, kTimeoutEmpty, (int)g)) { ok = false; break; }
+            mbar_expect_tx(&ctl.qdo_full[s], 2 * kQTile);
+            uint8_t* st = sQO + s * 2 * kQTile;
 #pragma unroll
-      for (int pn = 0; pn < NP; ++pn) {
-        tma_load_3d(sK + pn * kPanelBytes, &tmK, &kv_full, p.k_col0 + hkv * D + pn * 64, kv0, b);
-        tma_load_3d(sV + pn * kPanelBytes, &tmV, &kv_full, p.v_col0 + hkv * D + pn * 64, kv0, b);
-      }
-      for (int it = 0; it < n_iter; ++it) {
-        const int s = it % kStages;
-        const uint32_t ph = (it / kStages) & 1;
-        const int hq = hkv * group + it / n_i;
-        const int qi = i_begin + it % n_i;
-        if (!mbar_wait(&qdo_empty[s], ph ^ 1, &abort_flag, p.status, kTimeoutEmpty, it)) break;
-        mbar_expect_tx(&qdo_full[s], 2 * kTile);
+            for (int pn = 0; pn < NP; ++pn) {
+              tma_load_3d(st + pn * kQPanel, &tmQ, &ctl.qdo_full[s], p.q_col0 + hq * D + pn * 64, qi * 64, b);
+              tma_load_3d(st + kQTile + pn * kQPanel, &tmdO, &ctl.qdo_full[s], p.o_col0 + hq * D + pn * 64, qi * 64, b);
+            }
+            if (!kv_loaded) {   // behind the item's first block: its stage is free before the K / V tile is
+              const uint32_t kb = n % kKV;
+              if (!mbar_wait(&ctl.kv_empty[kb], ((n / kKV) & 1) ^ 1, &abort_flag, p.status, kTimeoutEmpty, 1000)) { ok = false; break; }
+              mbar_expect_tx(&ctl.kv_full[kb], 2 * kTile);
+              uint8_t* kv = sKV + kb * 2 * kTile;
 #pragma unroll
-        for (int pn = 0; pn < NP; ++pn) {
-          tma_load_3d(sQ + s * kTile + pn * kPanelBytes, &tmQ, &qdo_full[s],
-                      p.q_col0 + hq * D + pn * 64, qi * 128, b);
-          tma_load_3d(sdO + s * kTile + pn * kPanelBytes, &tmdO, &qdo_full[s],
-                      p.o_col0 + hq * D + pn * 64, qi * 128, b);
+              for (int pn = 0; pn < NP; ++pn) {
+                tma_load_3d(kv + pn * kPanelBytes, &tmK, &ctl.kv_full[kb], p.k_col0 + hkv * D + pn * 64, jb * 128, b);
+                tma_load_3d(kv + kTile + pn * kPanelBytes, &tmV, &ctl.kv_full[kb], p.v_col0 + hkv * D + pn * 64, jb * 128, b);
+              }
+              kv_loaded = true;
+            }
+          }
         }
+        ++n;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_st = make_idesc_bf16(128, 128, 0, 0);  // K/V (K-major) x Q/dO (K-major)
-      const uint32_t idesc_dkv = make_idesc_bf16(128, D, 0, 1);   // P^T/dS^T (K-major) x dO/Q (MN)
-      const uint32_t idesc_dq = make_idesc_bf16(128, D, 1, 1);    // dS^T as MN-major A x K (MN)
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV);
-      const uint32_t aPt = smem_u32(sPt), adSt = smem_u32(sdSt);
-      bool ok = mbar_wait(&kv_full, 0, &abort_flag, p.status, kTimeoutFull, -1);
-      trace_stamp(p.trace, cta_lin, 3);
-      // S^T = K Q^T and dP^T = V dO^T of block `it` (the Q/dO stage must have landed)
-      auto issue_scores = [&](int it) -> bool {
-        const int s = it % kStages;
-        const uint32_t ph = (it / kStages) & 1;
-        if (!mbar_wait(&qdo_full[s], ph, &abort_flag, p.status, kTimeoutFull, it)) return false;
+    // ======================= scores: S^T = K Q^T and dP^T = V dO^T =======================
+    // (both issuing warps stay converged and elect a lane; see the GEMM kernels)
+    const uint32_t idesc_st = make_idesc_bf16(128, 64, 0, 0);   // K / V (K-major) x Q / dO (K-major)
+    const uint32_t lo_k = smem_desc_lo(smem_u32(sKV), 16), lo_q = smem_desc_lo(smem_u32(sQO), 16);
+    uint32_t g = 0, n = 0, s = 0, ph = 0, bf = 0, bph = 0;
+    bool ok = true;
+    for (int k = 0; k < rounds && ok; ++k) {
+      const int w = item_at(k);
+      if (w < 0) break;
+      const uint32_t kb = n % kKV;
+      const int n_iter = (num_qb - first_block(w)) * group;
+      if (!mbar_wait_warp(&ctl.kv_full[kb], (n / kKV) & 1, &abort_flag, p.status, kTimeoutFull, 1001)) break;
+      ++n;
+      const uint32_t ak = lo_k + kb * (2 * kTile >> 4);
+      for (int it = 0; it < n_iter; ++it, ++g) {
+        if (!mbar_wait_warp(&ctl.qdo_full[s], ph, &abort_flag, p.status, kTimeoutFull, (int)g)) { ok = false; break; }
+        // the buffer's columns were last P^T and dQ^T of kBufs blocks ago: dQ^T is drained and the products are done
+        if (!mbar_wait_warp(&ctl.dq_read[bf], bph ^ 1, &abort_flag, p.status, kTimeoutFlag, 200) ||
+            !mbar_wait_warp(&ctl.ds_free[bf], bph ^ 1, &abort_flag, p.status, kTimeoutFlag, 201)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t aQ = smem_u32(sQ + s * kTile), adO = smem_u32(sdO + s * kTile);
+        const uint32_t bq = lo_q + s * (2 * kQTile >> 4), d = bf * 128;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k)
-          umma_bf16_ss(tmem_base + kColSt, desc_kmajor(aK, k), desc_kmajor(aQ, k), idesc_st,
-                       k > 0 ? 1u : 0u);
+          for (int j = 0; j < D / 16; ++j)
+            umma_bf16_ss(d, smem_desc(ak + ((j >> 2) * kPanelBytes + (j & 3) * 32) / 16),
+                         smem_desc(bq + ((j >> 2) * kQPanel + (j & 3) * 32) / 16), idesc_st, j > 0 ? 1u : 0u);
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k)
-          umma_bf16_ss(tmem_base + kColdPt, desc_kmajor(aV, k), desc_kmajor(adO, k), idesc_st,
-                       k > 0 ? 1u : 0u);
-        umma_commit(&s_full);
-        return true;
-      };
-      if (ok && n_iter > 0) ok = issue_scores(0);
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const int s = it % kStages;
-        const int qb = it % kDQB;
-        if (!mbar_wait(&p_full, it & 1, &abort_flag, p.status, kTimeoutFlag, it)) { ok = false; break; }
-        tc_fence_after();
-        trace_stamp(p.trace, cta_lin, 8 + it * 6 + 5);
-        // S^T / dP^T of this block are consumed. With a dQ accumulator of its own the next
-        // block's scores can go first (its exponentials then overlap the MMAs below), provided
-        // its Q/dO stage has landed; otherwise they follow the gradient MMAs.
-        bool scores_issued = (it + 1 >= n_iter);
-        if (!kAliasdQ && !scores_issued) {
-          const int s1 = (it + 1) % kStages;
-          if (mbar_try_wait(&qdo_full[s1], ((it + 1) / kStages) & 1)) {
-            ok = issue_scores(it + 1);
-            scores_issued = true;
-          }
+          for (int j = 0; j < D / 16; ++j)
+            umma_bf16_ss(d + 64, smem_desc(ak + (kTile + (j >> 2) * kPanelBytes + (j & 3) * 32) / 16),
+                         smem_desc(bq + (kQTile + (j >> 2) * kQPanel + (j & 3) * 32) / 16), idesc_st, j > 0 ? 1u : 0u);
+          umma_commit(&ctl.s_full[bf]);
         }
-        const uint32_t aQ = smem_u32(sQ + s * kTile), adO = smem_u32(sdO + s * kTile);
-        // dV += P^T dO ; dK += dS^T Q   (contraction over the 128 query rows)
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_bf16_ss(tmem_base + kColdV, desc_kmajor(aPt, k), desc_mnmajor(adO, k), idesc_dkv,
-                       (it > 0 || k > 0) ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_bf16_ss(tmem_base + kColdK, desc_kmajor(adSt, k), desc_mnmajor(aQ, k), idesc_dkv,
-                       (it > 0 || k > 0) ? 1u : 0u);
-        // dQ = dS K  (contraction over the 128 key rows; dS^T tile read as an MN-major A)
-        if (!kAliasdQ && it >= kDQB) {
-          if (!mbar_wait(&dq_read[qb], ((it / kDQB) - 1) & 1, &abort_flag, p.status, kTimeoutFlag, 200 + it)) { ok = false; break; }
-          tc_fence_after();
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_bf16_ss(tmem_base + kColdQ + qb * D, desc_mnmajor(adSt, k), desc_mnmajor(aK, k),
-                       idesc_dq, k > 0 ? 1u : 0u);
-        umma_commit(&qdo_empty[s]);
-        umma_commit(&pds_free);
-        umma_commit(&dq_full[qb]);
-        if (it + 1 == n_iter) umma_commit(&acc_full);
-        if (!scores_issued) {
-          if (kAliasdQ) {
-            // dQ shares the S^T columns: the next scores wait until dQ has been drained
-            if (!mbar_wait(&dq_read[0], it & 1, &abort_flag, p.status, kTimeoutFlag, 300 + it)) { ok = false; break; }
-            tc_fence_after();
-          }
-          ok = issue_scores(it + 1);
-        }
+        __syncwarp();
+        if (++s == kStages) { s = 0; ph ^= 1; }
+        if (++bf == kBufs) { bf = 0; bph ^= 1; }
       }
     }
-  } else if (warp < 10) {
-    // ---------------- compute warps: one key row and half of the columns per thread --------
-    const int quad = warp & 3;
-    const int chalf = (warp - 2) >> 2;  // which half of the columns this warp handles
-    const int row = quad * 32 + lane;   // key row inside the block
-    const int kv_idx = kv0 + row;
-    const int ctid = threadIdx.x - 64;  // 0..255; the first 128 also stage lse / delta
-    const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
+  } else if (warp == 2) {
+    // ======================= gradients: dV += P^T dO, dK += dS^T Q, dQ^T = K^T dS^T =======================
+    const uint32_t idesc_dkv = make_idesc_bf16(128, D, 0, 1);   // P^T (TMEM) / dS^T (K-major) x dO / Q (MN)
+    const uint32_t idesc_dq = make_idesc_bf16(128, 64, 1, 1);   // K as MN-major A x dS^T (MN)
+    const uint32_t lo_kmn = smem_desc_lo(smem_u32(sKV), kPanelBytes), lo_qmn = smem_desc_lo(smem_u32(sQO), kQPanel);
+    const uint32_t lo_dsmn = smem_desc_lo(smem_u32(sdS), kDsBytes);
+    uint32_t g = 0, n = 0, s = 0, ph = 0, bf = 0, bph = 0;
+    bool ok = true;
+    for (int k = 0; k < rounds && ok; ++k) {
+      const int w = item_at(k);
+      if (w < 0) break;
+      const uint32_t kb = n % kKV;
+      const int n_iter = (num_qb - first_block(w)) * group;
+      if (!mbar_wait_warp(&ctl.kv_full[kb], (n / kKV) & 1, &abort_flag, p.status, kTimeoutFull, 1002)) break;
+      if (!mbar_wait_warp(&ctl.acc_empty, (n & 1) ^ 1, &abort_flag, p.status, kTimeoutTmemEmpty, 1003)) break;
+      ++n;
+      const uint32_t ak = lo_kmn + kb * (2 * kTile >> 4);
+      for (int it = 0; it < n_iter; ++it, ++g) {
+        if (!mbar_wait_warp(&ctl.qdo_full[s], ph, &abort_flag, p.status, kTimeoutFull, (int)g) ||
+            !mbar_wait_warp(&ctl.pds_full[bf], bph, &abort_flag, p.status, kTimeoutFlag, (int)g)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t bq = lo_qmn + s * (2 * kQTile >> 4);
+        const uint32_t bds = lo_dsmn + bf * (kDsBytes >> 4);
+        const uint32_t acc = it > 0 ? 1u : 0u;
+        // kCols columns of TMEM hold P^T and dS^T of kCols queries, half of them each, as bf16 pairs
+        auto pcol = [](int j) -> uint32_t { return (uint32_t)(kCols == 16 ? j * 16 : (j >> 1) * 32 + (j & 1) * 8); };
+        if (elect_one()) {
+          // dQ^T first: its drain is what the scores of two blocks on wait for. Contraction over the 128 key rows.
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            umma_bf16_ss(bf * 128 + 64, smem_desc(ak + j * 128), smem_desc(bds + j * 128), idesc_dq, j > 0 ? 1u : 0u);
+          umma_commit(&ctl.dq_full[bf]);
+          // contraction over the 64 query rows
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma_bf16_ts(kColV, bf * 128 + pcol(j), smem_desc(bq + (kQTile + j * 2048) / 16),
+                         idesc_dkv, j > 0 ? 1u : acc);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma_bf16_ts(kColK, bf * 128 + pcol(j) + kCols / 2, smem_desc(bq + j * 128), idesc_dkv,
+                         j > 0 ? 1u : acc);
+          umma_commit(&ctl.qdo_empty[s]);
+          umma_commit(&ctl.ds_free[bf]);   // P^T and dS^T of this buffer have been read
+          if (it + 1 == n_iter) {
+            umma_commit(&ctl.kv_empty[kb]);
+            umma_commit(&ctl.acc_full);
+          }
+        }
+        __syncwarp();
+        if (++s == kStages) { s = 0; ph ^= 1; }
+        if (++bf == kBufs) { bf = 0; bph ^= 1; }
+      }
+    }
+  } else if (warp >= 4 && warp < 4 + 8 * kGroups) {
+    // ---------------- compute warps: group 0 takes the even blocks, group 1 the odd ones --------
+    // (a block's chain of waits, TMEM reads and stores takes a group about 1900 cycles with two thirds of its issue
+    // slots empty: sixteen warps on one block gained nothing, two groups on two blocks overlap)
+    const int grp = (warp - 4) >> 3;
+    const int quad = warp & 3, chalf = ((warp - 4) >> 2) & 1;
+    const int row = quad * 32 + lane;
+    const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
     const float c = p.scale * 1.4426950408889634f;
     const float l2e = 1.4426950408889634f;
-    bool ok = true;
-
-    // lse / delta of query block `it` go to shared memory one iteration ahead: the global loads
-    // are issued at the top of iteration it-1 and stored at its end, so the wait on stat_full
-    // at the top of iteration `it` normally finds the phase complete.
+    float* my_lse = ctl.neg_lse[warp - 4];
+    float* my_delta = ctl.neg_delta[warp - 4];
+    // position in the CTA's sequence of blocks
+    struct Pos {
+      int k, w, b, hkv, hq, qi, i0;
+    };
+    auto enter = [&](Pos& q, int k) {
+      q.k = k;
+      q.w = item_at(k);
+      if (q.w >= 0) {
+        const int hb = q.w % n_heads_b;
+        q.hkv = hb % p.Hkv;
+        q.b = hb / p.Hkv;
+        q.hq = q.hkv * group;
+        q.i0 = q.qi = first_block(q.w);
+      }
+    };
+    auto advance = [&](Pos& q) {
+      if (q.w < 0) return;
+      if (++q.qi < num_qb) return;
+      q.qi = q.i0;
+      if (++q.hq < (q.hkv + 1) * group) return;
+      enter(q, q.k + 1);
+    };
+    // lse / delta of the warp's 32 columns, one (own) block ahead; queries past the end get lse = +inf, i.e. P = 0
+    // (raw values: arithmetic on them would wait for the loads here, a block early)
     float st_l = 0.f, st_d = 0.f;
-    auto stat_load = [&](int it) {
-      if (ctid < 128 && it < n_iter) {
-        const int hq = hkv * group + it / n_i;
-        const int q = (i_begin + it % n_i) * 128 + ctid;
-        const long long off = ((long long)b * p.Hq + hq) * p.T + q;
-        st_l = (q < p.T) ? p.lse[off] * l2e : 0.f;
-        st_d = (q < p.T) ? p.delta[off] : 0.f;
+    auto stat_load = [&](const Pos& z) {
+      st_l = INFINITY;
+      st_d = 0.f;
+      const int q = z.qi * 64 + chalf * 32 + lane;
+      if (z.w >= 0 && q < p.T) {
+        const long long off = ((long long)z.b * p.Hq + z.hq) * p.T + q;
+        st_l = p.lse[off];
+        st_d = p.delta[off];
       }
     };
-    auto stat_store = [&](int it) {
-      if (ctid < 128 && it < n_iter) {
-        s_lse[it & 1][ctid] = st_l;
-        s_delta[it & 1][ctid] = st_d;
-        mbar_arrive(&stat_full);
+    Pos cur, ahead;
+    enter(cur, 0);
+    if (grp == 1) advance(cur);
+    ahead = cur;
+    stat_load(ahead);
+    uint32_t bf = grp, bph = 0;   // the block's buffer and its phase
+    int stored = 0;   // items whose dV / dK this warp has stored (head_dim 128)
+    bool ok = true;
+    while (true) {
+      if (kBufs == 2) {
+        // items that lie behind: all MMAs into dV / dK have completed once acc_full fires
+        while (ok && item_at(stored) >= 0 && stored < cur.k) {
+          const int w = item_at(stored), hb = w % n_heads_b;
+          ok = store_grads(quad, chalf * (D / 64), (chalf + 1) * (D / 64), (uint32_t)stored, w / n_heads_b, hb % p.Hkv, hb / p.Hkv, nullptr);
+          ++stored;
+        }
       }
-    };
-    stat_load(0);
-    stat_store(0);
-
-    for (int it = 0; it < n_iter; ++it) {
-      const int qbase = (i_begin + it % n_i) * 128;
-      const float* lse_s = s_lse[it & 1];
-      const float* delta_s = s_delta[it & 1];
-      stat_load(it + 1);
-      if (!mbar_wait_warp(&stat_full, it & 1, &abort_flag, p.status, kTimeoutFlag, 500 + it)) { ok = false; break; }
-      if (!mbar_wait_warp(&s_full, it & 1, &abort_flag, p.status, kTimeoutTmemFull, it)) { ok = false; break; }
-      tc_fence_after();
-      if (tracer) trace_stamp(p.trace, cta_lin, 8 + it * 6 + 0);
-      const bool need_mask = (p.causal && (qbase < kv0 + 127)) || (qbase + 128 > p.T) ||
-                             (kv0 + 128 > p.T);
-      // Both variants are straight-line code (the mask is a select, not a branch), so that the
-      // 32 independent exp / multiply chains of a chunk interleave.
-      auto chunk = [&](auto masked_tag, int cc, float (&pt)[32], float (&ds)[32]) {
-        constexpr bool kMasked = decltype(masked_tag)::value;
-        const int col0 = chalf * 64 + cc * 32;
-        uint32_t rs[32], rp[32];
-        tmem_ld_32x32(t_lane + kColSt + col0, rs);
-        tmem_ld_32x32(t_lane + kColdPt + col0, rp);
-        tmem_ld_wait();
+      if (!ok || cur.w < 0) break;
+      const int kv_idx = cur.w / n_heads_b * 128 + row;
+      __syncwarp();   // every lane has read the previous block's values
+      my_lse[lane] = -st_l * l2e;
+      my_delta[lane] = -st_d;
+      __syncwarp();
 #pragma unroll
-        for (int i4 = 0; i4 < 8; ++i4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(&lse_s[col0 + 4 * i4]);
-          const float4 d4 = *reinterpret_cast<const float4*>(&delta_s[col0 + 4 * i4]);
+      for (int i = 0; i < kGroups; ++i) advance(ahead);
+      stat_load(ahead);
+      if (!mbar_wait_warp(&ctl.s_full[bf], bph, &abort_flag, p.status, kTimeoutTmemFull, (int)bf)) break;
+      tc_fence_after();
+      // (the scores waited for the products that last read this buffer, its dS^T tile among them)
+      uint8_t* rowp = sdS + bf * kDsBytes + row * 128;
+#pragma unroll
+      for (int sub = 0; sub < 32 / kCols; ++sub) {
+        const uint32_t col = bf * 128 + chalf * 32 + sub * kCols;
+        uint32_t rs[kCols], rp[kCols];
+        tmem_ld_cols(t_lane + col, rs);
+        tmem_ld_cols(t_lane + col + 64, rp);
+        tmem_ld_wait();
+        // Queries below the key row (causal) and key rows past the end have P = 0: their scores become -inf. (A
+        // second, masked copy of the block below ran twice an item, each time from a cold instruction cache, and took
+        // 2000 cycles longer than the plain one.)
+        const int lim = p.causal ? kv_idx - (cur.qi * 64 + chalf * 32 + sub * kCols) : 0;   // columns below it are dead
+        const bool past = kv_idx >= p.T;
+        if (__any_sync(0xffffffffu, (lim > 0) | past)) {
+          const uint32_t live = (past || lim >= kCols) ? 0u : lim <= 0 ? 0xffffffffu : 0xffffffffu << lim;
+#pragma unroll
+          for (int i = 0; i < kCols; ++i) rs[i] = (live & (1u << i)) ? rs[i] : 0xff800000u;
+        }
+        uint32_t pw[kCols];   // P^T as bf16 pairs, then dS^T
+#pragma unroll
+        for (int i4 = 0; i4 < kCols / 4; ++i4) {
+          const float4 l4 = *reinterpret_cast<const float4*>(&my_lse[sub * kCols + 4 * i4]);
+          const float4 d4 = *reinterpret_cast<const float4*>(&my_delta[sub * kCols + 4 * i4]);
           const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
           const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
+          float e[4], ds[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int i = 4 * i4 + u;
-            float e = exp2f(fmaf(__uint_as_float(rs[i]), c, -ls[u]));
-            if (kMasked) {
-              const int q = qbase + col0 + i;
-              const bool dead = (q >= p.T) | (kv_idx >= p.T) | ((p.causal != 0) & (kv_idx > q));
-              e = dead ? 0.f : e;
-            }
-            pt[i] = e;
-            ds[i] = e * (__uint_as_float(rp[i]) - dl[u]);
+          for (int v = 0; v < 4; ++v) {
+            const int i = 4 * i4 + v;
+            e[v] = exp2f(fmaf(__uint_as_float(rs[i]), c, ls[v]));
+            ds[v] = e[v] * (__uint_as_float(rp[i]) + dl[v]);
           }
+          pw[2 * i4] = pack_bf16x2(e[0], e[1]);
+          pw[2 * i4 + 1] = pack_bf16x2(e[2], e[3]);
+          pw[kCols / 2 + 2 * i4] = pack_bf16x2(ds[0], ds[1]);
+          pw[kCols / 2 + 2 * i4 + 1] = pack_bf16x2(ds[2], ds[3]);
+          if (i4 & 1)   // eight columns of dS^T
+            *reinterpret_cast<uint4*>(rowp + (((chalf * 4 + sub * (kCols / 8) + (i4 >> 1)) ^ (row & 7)) << 4)) =
+                make_uint4(pw[kCols / 2 + 2 * i4 - 2], pw[kCols / 2 + 2 * i4 - 1], pw[kCols / 2 + 2 * i4],
+                           pw[kCols / 2 + 2 * i4 + 1]);
         }
-      };
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        float pt[32], ds[32];
-        if (need_mask) chunk(TrueTag{}, cc, pt, ds);
-        else chunk(FalseTag{}, cc, pt, ds);
-        if (tracer && cc == 0) trace_stamp(p.trace, cta_lin, 8 + it * 6 + 1);
-        if (cc == 0 && it > 0) {
-          // the gradient MMAs of the previous block read P^T / dS^T: they must have finished
-          if (!mbar_wait_warp(&pds_free, (it - 1) & 1, &abort_flag, p.status, kTimeoutFlag, 600 + it)) { ok = false; break; }
-        }
-        store_chunk_sw128(sPt, row, chalf * 64 + cc * 32, pt);
-        store_chunk_sw128(sdSt, row, chalf * 64 + cc * 32, ds);
+        tmem_st_cols(t_lane + col, pw);
       }
-      if (!ok) break;
       fence_proxy_async_smem();
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full);
-      if (tracer) trace_stamp(p.trace, cta_lin, 8 + it * 6 + 2);
-      if (ctid < 128 && it + 1 < n_iter) {
-        // Every compute warp has passed its wait on stat_full(it) once p_full(it) completes;
-        // arriving for the next phase any earlier could complete it before a slow warp looked
-        // at this one. The scores of block it+1 need p_full(it) as well, so this costs nothing.
-        if (!mbar_wait_warp(&p_full, it & 1, &abort_flag, p.status, kTimeoutFlag, 800 + it)) { ok = false; break; }
-        stat_store(it + 1);
+      if (lane == 0) mbar_arrive(&ctl.pds_full[bf]);
+#pragma unroll
+      for (int i = 0; i < kGroups; ++i) {
+        advance(cur);
+        if (++bf == kBufs) { bf = 0; bph ^= 1; }
       }
     }
-    // all MMAs into dV / dK have completed once acc_full fires
-    if (ok && n_iter > 0)
-      ok = mbar_wait_warp(&acc_full, 0, &abort_flag, p.status, kTimeoutTmemFull, 700);
-    tc_fence_after();
-    // tcgen05.ld is warp-collective: the condition around it must be warp-uniform; only the
-    // global stores are predicated per row.
-    const bool warp_ok = __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
-    const bool row_ok = kv_idx < p.T;
-    if (tracer) trace_stamp(p.trace, cta_lin, 4);
-    if (warp_ok && n_iter > 0) {
-      __nv_bfloat16* dk = p.dK + ((long long)b * p.T + kv_idx) * p.ld_dk + p.dk_col0 + hkv * D;
-      __nv_bfloat16* dv = p.dV + ((long long)b * p.T + kv_idx) * p.ld_dv + p.dv_col0 + hkv * D;
-#pragma unroll
-      for (int c2 = 0; c2 < D / 64; ++c2) {
-        const int cc = chalf * (D / 64) + c2;
-        uint32_t r[32];
-        tmem_ld_32x32(t_lane + kColdV + cc * 32, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint4 q;
-          q.x = pack_bf16x2(__uint_as_float(r[8 * i + 0]), __uint_as_float(r[8 * i + 1]));
-          q.y = pack_bf16x2(__uint_as_float(r[8 * i + 2]), __uint_as_float(r[8 * i + 3]));
-          q.z = pack_bf16x2(__uint_as_float(r[8 * i + 4]), __uint_as_float(r[8 * i + 5]));
-          q.w = pack_bf16x2(__uint_as_float(r[8 * i + 6]), __uint_as_float(r[8 * i + 7]));
-          if (row_ok) reinterpret_cast<uint4*>(dv + cc * 32)[i] = q;
-        }
-        tmem_ld_32x32(t_lane + kColdK + cc * 32, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint4 q;
-          q.x = pack_bf16x2(__uint_as_float(r[8 * i + 0]) * p.scale, __uint_as_float(r[8 * i + 1]) * p.scale);
-          q.y = pack_bf16x2(__uint_as_float(r[8 * i + 2]) * p.scale, __uint_as_float(r[8 * i + 3]) * p.scale);
-          q.z = pack_bf16x2(__uint_as_float(r[8 * i + 4]) * p.scale, __uint_as_float(r[8 * i + 5]) * p.scale);
-          q.w = pack_bf16x2(__uint_as_float(r[8 * i + 6]) * p.scale, __uint_as_float(r[8 * i + 7]) * p.scale);
-          if (row_ok) reinterpret_cast<uint4*>(dk + cc * 32)[i] = q;
-        }
-      }
-    } else if (warp_ok && row_ok && n_iter == 0) {
-      // no query block attends to this key block: gradients are zero
-      __nv_bfloat16* dk = p.dK + ((long long)b * p.T + kv_idx) * p.ld_dk + p.dk_col0 + hkv * D;
-      __nv_bfloat16* dv = p.dV + ((long long)b * p.T + kv_idx) * p.ld_dv + p.dv_col0 + hkv * D;
-      for (int i = chalf * (D / 16); i < (chalf + 1) * (D / 16); ++i) {
-        reinterpret_cast<uint4*>(dk)[i] = make_uint4(0, 0, 0, 0);
-        reinterpret_cast<uint4*>(dv)[i] = make_uint4(0, 0, 0, 0);
-      }
-    }
-  } else {
-    // ---------------- dQ drain warps: one query row per thread ----------------
+  } else if (warp >= 4 + 8 * kGroups) {
+    // ---------------- dQ drain warps: 32 values of head_dim (one per lane), 64 queries --------
     const int quad = warp & 3;
-    const int row = quad * 32 + lane;
     const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const bool elected = (threadIdx.x == 320);  // issues the TMA reductions; also the tracer
-    uint8_t* my_row = sDQ + row * 128;
-    int u = 0;  // staging-tile uses so far (D / 64 per query block)
+    float* stg = reinterpret_cast<float*>(sDQ + quad * 2 * kDqBytes);
+    uint32_t n = 0, bf = 0, bph = 0;
     bool ok = true;
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int qb = it % kDQB;
-      if (!mbar_wait_warp(&dq_full[qb], (it / kDQB) & 1, &abort_flag, p.status, kTimeoutTmemFull, 100 + it)) break;
-      tc_fence_after();
-      if (elected) trace_stamp(p.trace, cta_lin, 8 + it * 6 + 3);
-      const int hq = hkv * group + it / n_i;
-      const int q0 = (i_begin + it % n_i) * 128;
+    for (int k = 0; k < rounds && ok; ++k) {
+      const int w = item_at(k);
+      if (w < 0) break;
+      const int jb = w / n_heads_b, hb = w - jb * n_heads_b;
+      const int hkv = hb % p.Hkv, b = hb / p.Hkv;
+      const int i0 = first_block(w);
+      for (int hq = hkv * group; quad < kDrain && hq < (hkv + 1) * group && ok; ++hq) {
+        for (int qi = i0; qi < num_qb; ++qi) {
+          if (!mbar_wait_warp(&ctl.dq_full[bf], bph, &abort_flag, p.status, kTimeoutTmemFull, 100)) { ok = false; break; }
+          tc_fence_after();
+          // 64 queries at once where registers allow it, so that the columns are handed back early
+          constexpr int kAtOnce = (kGroups == 1) ? 2 : 1;
+          uint32_t r[kAtOnce][32];
 #pragma unroll
-      for (int h2 = 0; h2 < D / 64; ++h2, ++u) {
-        uint32_t r[2][32];
-        tmem_ld_32x32(t_lane + kColdQ + qb * D + h2 * 64, r[0]);
-        tmem_ld_32x32(t_lane + kColdQ + qb * D + h2 * 64 + 32, r[1]);
-        tmem_ld_wait();
-        if (h2 == D / 64 - 1) {
-          // the accumulator is in registers: hand its TMEM columns back right away
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&dq_read[qb]);
-        }
-        // the previous reduction must have finished reading the staging tile
-        if (u > 0 && !mbar_wait_warp(&stage_free, (u - 1) & 1, &abort_flag, p.status, kTimeoutFlag, 900 + it)) { ok = false; break; }
+          for (int h = 0; h < 2; ++h) {
+            if (h % kAtOnce == 0) {
 #pragma unroll
-        for (int pn = 0; pn < 2; ++pn) {
+              for (int i = 0; i < kAtOnce; ++i) tmem_ld_32x32(t_lane + bf * 128 + 64 + (h + i) * 32, r[i]);
+              tmem_ld_wait();
+              if (h + kAtOnce == 2) {   // dQ^T is in registers: its columns are free
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ctl.dq_read[bf]);
+              }
+            }
+            if (lane == 0) bulk_wait_group_read1();   // at most the other half's reduction still reads its tile
+            __syncwarp();
+            float* t = stg + h * (kDqBytes / 4);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float4 v;
-            v.x = __uint_as_float(r[pn][4 * j + 0]) * p.scale;
-            v.y = __uint_as_float(r[pn][4 * j + 1]) * p.scale;
-            v.z = __uint_as_float(r[pn][4 * j + 2]) * p.scale;
-            v.w = __uint_as_float(r[pn][4 * j + 3]) * p.scale;
-            *reinterpret_cast<float4*>(my_row + pn * kPanelBytes + ((j ^ (row & 7)) << 4)) = v;
+            for (int q = 0; q < 32; ++q) t[q * 32 + lane] = __uint_as_float(r[h % kAtOnce][q]) * p.scale;
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              // queries past T are clipped by the tensor map (3-D: columns, rows of one batch, batch)
+              if (qi * 64 + h * 32 < p.T)
+                tma_reduce_add_3d(&tmdQ, t, p.dq_col0 + hq * D + quad * 32, qi * 64 + h * 32, b);
+              bulk_commit_group();
+            }
           }
+          if (++bf == kBufs) { bf = 0; bph ^= 1; }
         }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&dq_staged);
-        if (elected) {
-          if (!mbar_wait(&dq_staged, u & 1, &abort_flag, p.status, kTimeoutFlag, 1000 + it)) { ok = false; }
-          else {
-            // rows past T are clipped by the tensor map (3-D: columns, rows of one batch, batch)
-#pragma unroll
-            for (int pn = 0; pn < 2; ++pn)
-              tma_reduce_add_3d(&tmdQ, sDQ + pn * kPanelBytes,
-                                p.dq_col0 + hq * D + h2 * 64 + pn * 32, q0, b);
-            bulk_commit_group();
-            bulk_wait_group_read0();
-            mbar_arrive(&stage_free);
-          }
-        }
-        ok = __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
-        if (!ok) break;
       }
-      if (elected) trace_stamp(p.trace, cta_lin, 8 + it * 6 + 4);
+      if (kBufs == 3 && ok) {
+        if (lane == 0) bulk_wait_group_read0();   // the staging tiles are free
+        __syncwarp();
+        ok = store_grads(quad, 0, D / 32, n++, jb, hkv, b, sDQ + quad * 2 * kDqBytes);
+      }
     }
-    if (elected) bulk_wait_group0();  // reductions in flight finish before the CTA retires
+    if (lane == 0) bulk_wait_group0();  // reductions in flight finish before the CTA retires
   }
 
-  if (tracer) trace_stamp(p.trace, cta_lin, 5);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
     tmem_dealloc(tmem_base, kTmemCols);
   }
-  if (tracer) trace_stamp(p.trace, cta_lin, 6);
 }
 
 static long long* g_attn_trace = nullptr;
@@ -1332,7 +1407,7 @@ static int make_tmap_btc(CUtensorMap* out, const void* base, int B, int T, long 
   return (r == CUDA_SUCCESS) ? 0 : (int)r;
 }
 
-// fp32 accumulator [B*T, ld] viewed as [B][T][ld]; boxes of 32 columns x 128 rows, 128-byte swizzle
+// fp32 accumulator [B*T, ld] viewed as [B][T][ld]; boxes of 32 columns x 32 rows
 static int make_tmap_f32_btc(CUtensorMap* out, const void* base, int B, int T, long long ld) {
   EncodeTiledFn fn = attn_encode_fn();
   if (fn == nullptr) return -1;
@@ -1340,10 +1415,10 @@ static int make_tmap_f32_btc(CUtensorMap* out, const void* base, int B, int T, l
   if (ld % 4 || ((uintptr_t)base & 15)) return -2;
   cuuint64_t dims[3] = {(cuuint64_t)ld, (cuuint64_t)T, (cuuint64_t)B};
   cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)ld * 4 * (cuuint64_t)T};
-  cuuint32_t box[3] = {32, 128, 1};
+  cuuint32_t box[3] = {32, 32, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return (r == CUDA_SUCCESS) ? 0 : (int)r;
 }
@@ -1434,8 +1509,8 @@ MMJ_API int mmj_attn_fwd(const void* q, long long ldq, int q_col0, const void* k
   return (int)cudaGetLastError();
 }
 
-// Install (or clear, with nullptr) the timeline buffer of the attention kernels: int64
-// [ctas * 64], written by whichever of them is launched next. Launches whose grid has more CTAs than `ctas` leave it untouched.
+// Install (or clear, with nullptr) the timeline buffer of the forward kernels: int64 [ctas * 64], written by whichever of
+// them is launched next. Launches whose grid has more CTAs than `ctas` leave it untouched.
 MMJ_API int mmj_attn_set_trace(void* buf, long long ctas) {
   g_attn_trace = reinterpret_cast<long long*>(buf);
   g_attn_trace_ctas = buf ? ctas : 0;
@@ -1457,10 +1532,10 @@ MMJ_API int mmj_attn_bwd(const void* q, long long ldq, int q_col0, const void* k
   if (ld_dk % 8 || ld_dv % 8 || dk_col0 % 8 || dv_col0 % 8 || ld_dq % 4 || dq_col0 % 4) return -12;
   CUtensorMap tq, tk, tv, tdo;
   int rc;
-  if ((rc = make_tmap_btc(&tq, q, B, T, ldq, ldq))) return rc;
+  if ((rc = make_tmap_btc(&tq, q, B, T, ldq, ldq, 64))) return rc;
   if ((rc = make_tmap_btc(&tk, k, B, T, ldk, ldk))) return rc;
   if ((rc = make_tmap_btc(&tv, v, B, T, ldv, ldv))) return rc;
-  if ((rc = make_tmap_btc(&tdo, dO, B, T, lddo, lddo))) return rc;
+  if ((rc = make_tmap_btc(&tdo, dO, B, T, lddo, lddo, 64))) return rc;
   CUtensorMap tdq;
   if (dq_col0 % 4) return -13;
   if ((rc = make_tmap_f32_btc(&tdq, dQ_accum, B, T, ld_dq))) return rc;
@@ -1484,28 +1559,24 @@ MMJ_API int mmj_attn_bwd(const void* q, long long ldq, int q_col0, const void* k
   p.dK = (__nv_bfloat16*)dK; p.ld_dk = ld_dk; p.dk_col0 = dk_col0;
   p.dV = (__nv_bfloat16*)dV; p.ld_dv = ld_dv; p.dv_col0 = dv_col0;
   p.status = status;
-  p.trace = g_attn_trace;
-  dim3 grid((unsigned)(((T + 127) / 128) * Hkv * B));
-  if (g_attn_trace && (long long)grid.x > g_attn_trace_ctas) p.trace = nullptr;
-  static bool attr64 = false, attr128 = false;
-  if (D == 64) {
-    // K,V + 3x(Q,dO) + P^T,dS^T + dQ staging = 224 KB of tiles; the control block and the alignment
-    // padding take what is left of the 227 KB a CTA may have (the kernel checks that they fit)
-    const int smem = 232448;
-    if (!attr64) {
-      cudaFuncSetAttribute(attn_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      attr64 = true;
-    }
-    launch_pdl(attn_bwd_kernel<64>, grid, dim3(kAttnBwdThreads), (size_t)smem, (cudaStream_t)stream, tq, tk, tv,
-               tdo, tdq, p);
-  } else {
-    const int smem = 232448;  // 224 KB of tiles as well: K,V + Q,dO + P^T,dS^T + dQ staging
-    if (!attr128) {
-      cudaFuncSetAttribute(attn_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      attr128 = true;
-    }
-    launch_pdl(attn_bwd_kernel<128>, grid, dim3(kAttnBwdThreads), (size_t)smem, (cudaStream_t)stream, tq, tk, tv,
-               tdo, tdq, p);
+  const long long n_items = (long long)((T + 127) / 128) * Hkv * B;
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   }
+  const dim3 grid((unsigned)(n_items < sms ? n_items : sms));
+  // head_dim 128: 224 KB of tiles, the control block and the alignment padding take what is left of the 227 KB a CTA
+  // may have (the kernel checks that they fit); head_dim 64 needs 208 KB of tiles
+  const int smem = 232448;
+  static bool attr64 = false, attr128 = false;
+  bool& attr = (D == 64) ? attr64 : attr128;
+  auto* kernel = (D == 64) ? &attn_bwd_kernel<64> : &attn_bwd_kernel<128>;
+  if (!attr) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    attr = true;
+  }
+  launch_pdl(kernel, grid, dim3(D == 64 ? BwdCfg<64>::kThreads : BwdCfg<128>::kThreads), (size_t)smem, (cudaStream_t)stream, tq, tk, tv, tdo, tdq, p);
   return (int)cudaGetLastError();
 }

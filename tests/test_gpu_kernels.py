@@ -356,3 +356,26 @@ def test_sq_norm_edges(dtype, n, shift):
             found.zero_()
             ops.sq_norm(y, found_inf=found)
             assert int(found) == 1
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [
+    (1, 1, 1, 1, 64), (2, 63, 2, 2, 64), (1, 65, 4, 1, 64), (3, 129, 2, 1, 64),   # one block, its edges, a lone last one
+    (1, 1, 1, 1, 128), (2, 64, 2, 1, 128), (1, 191, 4, 1, 128), (1, 257, 2, 2, 128),
+    (40, 200, 8, 4, 64), (40, 130, 8, 4, 128),                                     # several items to a CTA
+])
+def test_attention_backward_block_edges(B, T, Hq, Hkv, D, causal):
+    """Blocks of 64 queries and 128 keys, the buffers of consecutive items, masked and ragged ones among them. The
+    products' operands are rounded to bf16 (2^-9 each, three in a row), far below the 1 % of the comparison."""
+    torch.manual_seed(11)
+    qkv = _rand(B * T, (Hq + 2 * Hkv) * D, grad=True)
+    dy = _rand(B * T, Hq * D)
+    (got,) = torch.autograd.grad(ops.attention_packed(qkv, B, T, Hq, Hkv, D, causal=causal), qkv, dy)
+    x = qkv.detach().float().requires_grad_()
+    v = x.view(B, T, Hq + 2 * Hkv, D).transpose(1, 2)
+    ref = _attn_ref(v[:, :Hq], v[:, Hq:Hq + Hkv], v[:, Hq + Hkv:], causal).transpose(1, 2).reshape(B * T, Hq * D)
+    (want,) = torch.autograd.grad(ref, x, dy.float())
+    for lo, hi in ((0, Hq), (Hq, Hq + Hkv), (Hq + Hkv, Hq + 2 * Hkv)):
+        if T > 1 or lo >= Hq + Hkv:     # with one key dQ and dK vanish
+            _close(got[:, lo * D:hi * D], want[:, lo * D:hi * D])
+    assert torch.isfinite(got).all()
