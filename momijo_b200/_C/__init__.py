@@ -37,6 +37,8 @@ _SIGS = {
     "mmj_swiglu_fwd": ([P, P, L, I, P], 1),
     "mmj_swiglu_bwd": ([P, P, P, L, I, P], 1),
     "mmj_rope": ([P, P, L, L, I, I, I, I, F, P], 1),
+    "mmj_rope_copy": ([P, P, P, L, L, I, I, I, I, P], 1),
+    "mmj_rope_grad": ([P, L, P, L, P, L, I, I, I, I, P], 1),
     "mmj_embedding_fwd": ([P, P, P, P, L, I, I, I, P], 1),
     "mmj_embedding_bwd": ([P, P, P, P, L, I, I, I, I, P], 2),
     "mmj_colsum_splits": ([I], 0),

@@ -480,7 +480,7 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_slot;
+  constexpr uint32_t tmem_base = 0;   // an allocation of all 512 columns starts at column 0
   pdl_wait();  // the set-up above touched no global memory
   pdl_trigger();
 
@@ -551,12 +551,14 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   } else if (warp == 1 || warp == 2) {
     // ======================= MMA issuers: warp 1 drives query tile 0, warp 2 tile 1 =======================
-    // (a single issuing thread spends about 1400 cycles per tile and key block on waits, descriptors,
-    // MMAs and commits; with one thread per tile the two tiles' chains no longer queue behind each other)
-    if (lane == 0) {
+    // (the warps stay converged and elect a lane to issue; one issuer for both tiles queued their chains behind each
+    // other)
+    {
       const int t = warp - 1;
       const uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);
       const uint32_t idesc_o = make_idesc_bf16(128, D, 0, 1);
+      const uint32_t lo_q = smem_desc_lo(smem_u32(sQ) + t * kQTile, 16), lo_k = smem_desc_lo(smem_u32(sK), 16);
+      const uint32_t lo_v = smem_desc_lo(smem_u32(sV), kKVPanel);
       uint32_t qn = 0;
       uint32_t pc[2] = {0, 0};  // P tiles consumed so far, per buffer
       uint32_t on = 0;
@@ -571,23 +573,24 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         auto issue_s = [&](int j) -> bool {
           const uint32_t c = kc + (uint32_t)j;
           const int s = c % KS;
-          if (!mbar_wait(&k_full[s], (c / KS) & 1, &abort_flag, p.status, kTimeoutFull, j)) return false;
+          if (!mbar_wait_warp(&k_full[s], (c / KS) & 1, &abort_flag, p.status, kTimeoutFull, j)) return false;
           tc_fence_after();
-          const uint32_t aQ = smem_u32(sQ + t * kQTile), aK = smem_u32(sK + s * kKVTile);
-          const uint32_t d = tmem_base + (uint32_t)(t * 128 + (j & 1) * 64);
+          if (elect_one()) {
+            const uint32_t d = (uint32_t)(t * 128 + (j & 1) * 64), bk = lo_k + s * (kKVTile >> 4);
 #pragma unroll
-          for (int k = 0; k < D / 16; ++k) {
-            // K tile: 64 rows, 64-column panels of 8 KiB
-            const uint64_t dk = make_smem_desc(aK + (uint32_t)(k >> 2) * kKVPanel + (uint32_t)(k & 3) * 32, 16, 1024);
-            umma_bf16_ss(d, desc_kmajor(aQ, k), dk, idesc_s, k > 0 ? 1u : 0u);
+            for (int k = 0; k < D / 16; ++k)
+              // K tile: 64 rows, 64-column panels of 8 KiB
+              umma_bf16_ss(d, smem_desc(lo_q + ((k >> 2) * kPanelBytes + (k & 3) * 32) / 16),
+                           smem_desc(bk + ((k >> 2) * kKVPanel + (k & 3) * 32) / 16), idesc_s, k > 0 ? 1u : 0u);
+            umma_commit(&s_full[t][j & 1]);
+            umma_commit(&k_empty[s]);   // this tile's share of the K block's release
+            if (j + 1 == nbt) umma_commit(&q_empty[t]);
           }
-          umma_commit(&k_empty[s]);   // this tile's share of the K block's release
-          if (j + 1 == nbt) umma_commit(&q_empty[t]);
-          umma_commit(&s_full[t][j & 1]);
+          __syncwarp();
           return true;
         };
         if (nbt > 0) {
-          if (!mbar_wait(&q_full[t], qn & 1, &abort_flag, p.status, kTimeoutFull, 400 + t)) { ok = false; break; }
+          if (!mbar_wait_warp(&q_full[t], qn & 1, &abort_flag, p.status, kTimeoutFull, 400 + t)) { ok = false; break; }
           ++qn;
           ok = issue_s(0);
           if (ok && nbt > 1) ok = issue_s(1);
@@ -598,30 +601,30 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (j >= nbt) {
             // a key block only the other tile reads: hand in this tile's share of its release, but only
             // once the block has been loaded (an earlier arrival would count for the stage's previous block)
-            if (!mbar_wait(&k_full[sv], (c / KS) & 1, &abort_flag, p.status, kTimeoutFull, 800 + j)) { ok = false; break; }
-            mbar_arrive(&k_empty[sv]);
-            if (!mbar_wait(&v_full[sv], (c / KS) & 1, &abort_flag, p.status, kTimeoutFull, 900 + j)) { ok = false; break; }
-            mbar_arrive(&v_empty[sv]);
+            if (!mbar_wait_warp(&k_full[sv], (c / KS) & 1, &abort_flag, p.status, kTimeoutFull, 800 + j)) { ok = false; break; }
+            if (lane == 0) mbar_arrive(&k_empty[sv]);
+            if (!mbar_wait_warp(&v_full[sv], (c / KS) & 1, &abort_flag, p.status, kTimeoutFull, 900 + j)) { ok = false; break; }
+            if (lane == 0) mbar_arrive(&v_empty[sv]);
             continue;
           }
           const int bf = j & 1;
-          if (!mbar_wait(&p_full[t][bf], pc[bf] & 1, &abort_flag, p.status, kTimeoutFlag, 500 + j)) { ok = false; break; }
-          ++pc[bf];
+          if (!mbar_wait_warp(&v_full[sv], (c / KS) & 1, &abort_flag, p.status, kTimeoutFull, 100 + j)) { ok = false; break; }
           if (j == 0 && on > 0) {
-            if (!mbar_wait(&o_free[t], (on - 1) & 1, &abort_flag, p.status, kTimeoutTmemEmpty, 600 + t)) { ok = false; break; }
+            if (!mbar_wait_warp(&o_free[t], (on - 1) & 1, &abort_flag, p.status, kTimeoutTmemEmpty, 600 + t)) { ok = false; break; }
           }
-          if (!mbar_wait(&v_full[sv], (c / KS) & 1, &abort_flag, p.status, kTimeoutFull, 100 + j)) { ok = false; break; }
+          if (!mbar_wait_warp(&p_full[t][bf], pc[bf] & 1, &abort_flag, p.status, kTimeoutFlag, 500 + j)) { ok = false; break; }
+          ++pc[bf];
           tc_fence_after();
-          const uint32_t aV = smem_u32(sV + sv * kKVTile);
-          const uint32_t aP = tmem_base + (uint32_t)(t * 128 + bf * 64);
+          if (elect_one()) {
+            const uint32_t bv = lo_v + sv * (kKVTile >> 4), aP = (uint32_t)(t * 128 + bf * 64);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            // V tile as an MN-major B operand: 16 key rows per step, 64-wide panels 8 KiB apart
-            const uint64_t dv = make_smem_desc(aV + (uint32_t)k * 2048, kKVPanel, 1024);
-            umma_bf16_ts(tmem_base + kColO + t * D, aP + k * 8, dv, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < 4; ++k)
+              // V tile as an MN-major B operand: 16 key rows per step, 64-wide panels 8 KiB apart
+              umma_bf16_ts(kColO + t * D, aP + k * 8, smem_desc(bv + k * 128), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+            umma_commit(&o_done[t][bf]);   // P_t(j) V_j has landed in O_t
+            umma_commit(&v_empty[sv]);
           }
-          umma_commit(&v_empty[sv]);
-          umma_commit(&o_done[t][bf]);   // P_t(j) V_j has landed in O_t
+          __syncwarp();
           if (j + 1 == nbt) ++on;
           if (j + 2 < nbt) ok = issue_s(j + 2);
         }

@@ -391,9 +391,12 @@ class _AttnPacked(torch.autograd.Function):
         ld = qkv.shape[1]
         qc, kc, vc = 0, Hq * D, (Hq + Hkv) * D
         if rope is not None:
-            qkv = qkv.clone()
-            rope_inplace(qkv, rope, qc, Hq, D, T, 1.0)
-            rope_inplace(qkv, rope, kc, Hkv, D, T, 1.0)
+            if qkv.data_ptr() % 16:      # a view at an odd offset: the copy below reads 16 bytes at a time
+                qkv = qkv.clone()
+            rotated = torch.empty_like(qkv)
+            _C.call("mmj_rope_copy", _C.ptr(qkv), _C.ptr(rotated), _C.ptr(rope), qkv.shape[0], ld, Hq + Hkv, Hq + 2 * Hkv, D, T,
+                    _C.current_stream())
+            qkv = rotated
         out = torch.empty((B * T, Hq * D), dtype=bf16, device=qkv.device)
         lse = torch.empty((B, Hq, T), dtype=torch.float32, device=qkv.device)
         st = _C.status_tensor(qkv.device)
@@ -421,11 +424,12 @@ class _AttnPacked(torch.autograd.Function):
                 _C.ptr(delta), _C.ptr(dq_acc), dq_acc.stride(0), 0, _C.ptr(dqkv), ld, kc,
                 _C.ptr(dqkv), ld, vc, B, T, Hq, Hkv, D, scale, int(causal), _C.ptr(st),
                 _C.current_stream())
-        _C.call("mmj_cast_f32_to_bf16_2d", _C.ptr(dq_acc), dq_acc.stride(0), _C.ptr(dqkv), ld,
-                B * T, Hq * D, _C.current_stream())
-        if ctx.rope is not None:
-            rope_inplace(dqkv, ctx.rope, qc, Hq, D, T, -1.0)
-            rope_inplace(dqkv, ctx.rope, kc, Hkv, D, T, -1.0)
+        if ctx.rope is None:
+            _C.call("mmj_cast_f32_to_bf16_2d", _C.ptr(dq_acc), dq_acc.stride(0), _C.ptr(dqkv), ld,
+                    B * T, Hq * D, _C.current_stream())
+        else:
+            _C.call("mmj_rope_grad", _C.ptr(dq_acc), dq_acc.stride(0), _C.ptr(dqkv), ld, _C.ptr(ctx.rope), B * T, Hq, Hkv,
+                    D, T, _C.current_stream())
         return dqkv, None, None, None, None, None, None, None, None
 
 

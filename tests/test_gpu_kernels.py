@@ -379,3 +379,23 @@ def test_attention_backward_block_edges(B, T, Hq, Hkv, D, causal):
         if T > 1 or lo >= Hq + Hkv:     # with one key dQ and dK vanish
             _close(got[:, lo * D:hi * D], want[:, lo * D:hi * D])
     assert torch.isfinite(got).all()
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [(2, 37, 2, 1, 64), (1, 130, 4, 4, 128), (3, 5, 6, 2, 128)])
+def test_attention_rotary_paths(B, T, Hq, Hkv, D):
+    """Rotation fused into the copy of the packed rows and into the gradient's cast, a misaligned input view among
+    them, against the differentiable rotation of the CPU path."""
+    torch.manual_seed(3)
+    n = B * T * (Hq + 2 * Hkv) * D
+    buf = _rand(n + 1)
+    tab = ops.rope_table(T, D, 10000.0, "cuda")
+    for shift in (0, 1):
+        qkv = buf[shift:shift + n].view(B * T, -1).detach().requires_grad_()
+        dy = _rand(B * T, Hq * D)
+        y = ops.attention_packed(qkv, B, T, Hq, Hkv, D, rope=tab)
+        (got,) = torch.autograd.grad(y, qkv, dy)
+        x = qkv.detach().float().cpu().requires_grad_()
+        yr = ops.attention_packed(x, B, T, Hq, Hkv, D, rope=tab.cpu())
+        (want,) = torch.autograd.grad(yr, x, dy.float().cpu())
+        _close(y, yr.cuda())
+        _close(got, want.cuda())
