@@ -401,25 +401,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // group of tile 0; warps 8..11 = softmax group of tile 1 (one query row per thread). A softmax group reads
 // its score tile from tensor memory, writes the probabilities back over the first columns of the same tile
 // as packed bf16 pairs, and the P V product takes them from there as its tensor-memory A operand: P never
-// touches shared memory. Three things keep the tensor core out of the groups' dependency chain:
+// touches shared memory. Three things keep the groups' dependency chain short:
 //   * each query tile has its own MMA-issuing thread (warps 1 and 2);
 //   * a key block is 64 keys and every query tile owns TWO score buffers in tensor memory
 //     (S_t[0], S_t[1], 64 columns each): the MMA thread issues S_t(j+1) before the group has finished
 //     block j, so a group that has stored P_t(j) finds S_t(j+1) waiting and starts on it at once;
 //     per key block the MMA thread does  [wait P_t(j)]  P_t(j) V_j -> O_t,  Q_t K_(j+2)^T -> S_t[j & 1];
-//   * probabilities are rounded to bf16 with integer arithmetic (add half an ulp, take the upper
-//     halves with one byte permute) instead of the conversion instruction, which shares the
-//     transcendental pipe with the exponentials.
+//   * the softmax is bound by issue (two warps per scheduler at 60 % of the slots): three-operand maxima, paired
+//     multiply-adds and sums and the paired conversion take 192 instructions for 64 scores where scalar ones and
+//     integer rounding took 352.
 // Tensor memory: S0[0] S0[1] S1[0] S1[1] | O0 | O1 = 256 + 2 D columns; P_t(j) overwrites the first 32
 // columns of S_t[j & 1] (64 probabilities as bf16 pairs). Every P_t(j) V_j commits to o_done[t][j & 1];
 // a group waits on it only before it rescales O_t (rare: the running maximum must have grown by more
 // than 2^8) and before the final normalisation.
-__device__ __forceinline__ uint32_t pack_bf16x2_halfup(float lo, float hi) {
-  // lo, hi >= 0 (probabilities): adding 0x8000 to the bit pattern rounds the upper 16 bits half-up
-  const uint32_t a = __float_as_uint(lo) + 0x8000u, b = __float_as_uint(hi) + 0x8000u;
-  return __byte_perm(a, b, 0x7632);
-}
-
 template <int D>
 __global__ void __launch_bounds__(384, 1)
 attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -680,11 +674,11 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          mx0 = fmaxf(mx0, __uint_as_float(s[i + 0]));
-          mx1 = fmaxf(mx1, __uint_as_float(s[i + 1]));
-          mx2 = fmaxf(mx2, __uint_as_float(s[i + 2]));
-          mx3 = fmaxf(mx3, __uint_as_float(s[i + 3]));
+        for (int i = 0; i < 64; i += 8) {
+          mx0 = fmax3(mx0, __uint_as_float(s[i + 0]), __uint_as_float(s[i + 1]));
+          mx1 = fmax3(mx1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+          mx2 = fmax3(mx2, __uint_as_float(s[i + 4]), __uint_as_float(s[i + 5]));
+          mx3 = fmax3(mx3, __uint_as_float(s[i + 6]), __uint_as_float(s[i + 7]));
         }
         const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
         if (tr && j < 6) trace_stamp(p.trace, blockIdx.x, 8 + 24 * t + 4 * j + 2);
@@ -713,22 +707,25 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
           }
         }
-        const float mc = m_used * c;
-        float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+        const f32x2 c2 = f2_pack(c, c), mc2 = f2_pack(-m_used * c, -m_used * c);
+        f32x2 sum0 = 0ull, sum1 = 0ull;   // two zeros each
         // 64 probabilities as bf16 pairs, packed in place: pair m lands in s[m], which the loop has
         // already consumed (it reads s[2m ...], never behind its writes)
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          const float e0 = exp2f(fmaf(__uint_as_float(s[2 * i + 0]), c, -mc));
-          const float e1 = exp2f(fmaf(__uint_as_float(s[2 * i + 1]), c, -mc));
-          const float e2 = exp2f(fmaf(__uint_as_float(s[2 * i + 2]), c, -mc));
-          const float e3 = exp2f(fmaf(__uint_as_float(s[2 * i + 3]), c, -mc));
-          sum0 += e0; sum1 += e1; sum2 += e2; sum3 += e3;
-          s[i + 0] = pack_bf16x2_halfup(e0, e1);
-          s[i + 1] = pack_bf16x2_halfup(e2, e3);
+          float e0, e1, e2, e3;
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(s[2 * i + 0]), __uint_as_float(s[2 * i + 1])), c2, mc2), e0, e1);
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(s[2 * i + 2]), __uint_as_float(s[2 * i + 3])), c2, mc2), e2, e3);
+          e0 = exp2f(e0); e1 = exp2f(e1); e2 = exp2f(e2); e3 = exp2f(e3);
+          sum0 = f2_add(sum0, f2_pack(e0, e1));
+          sum1 = f2_add(sum1, f2_pack(e2, e3));
+          s[i + 0] = pack_bf16x2(e0, e1);
+          s[i + 1] = pack_bf16x2(e2, e3);
         }
         tmem_st_32x32(t_lane + colS, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
-        l += (sum0 + sum1) + (sum2 + sum3);
+        float l0, l1;
+        f2_unpack(f2_add(sum0, sum1), l0, l1);
+        l += l0 + l1;
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -1179,8 +1176,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int quad = warp & 3, chalf = ((warp - 4) >> 2) & 1;
     const int row = quad * 32 + lane;
     const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
-    const float c = p.scale * 1.4426950408889634f;
     const float l2e = 1.4426950408889634f;
+    const f32x2 c2 = f2_pack(p.scale * l2e, p.scale * l2e);
     float* my_lse = ctl.neg_lse[warp - 4];
     float* my_delta = ctl.neg_delta[warp - 4];
     // position in the CTA's sequence of blocks
@@ -1268,16 +1265,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         uint32_t pw[kCols];   // P^T as bf16 pairs, then dS^T
 #pragma unroll
         for (int i4 = 0; i4 < kCols / 4; ++i4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(&my_lse[sub * kCols + 4 * i4]);
-          const float4 d4 = *reinterpret_cast<const float4*>(&my_delta[sub * kCols + 4 * i4]);
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
-          const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
+          const ulonglong2 l4 = *reinterpret_cast<const ulonglong2*>(&my_lse[sub * kCols + 4 * i4]);
+          const ulonglong2 d4 = *reinterpret_cast<const ulonglong2*>(&my_delta[sub * kCols + 4 * i4]);
           float e[4], ds[4];
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int i = 4 * i4 + v;
-            e[v] = exp2f(fmaf(__uint_as_float(rs[i]), c, ls[v]));
-            ds[v] = e[v] * (__uint_as_float(rp[i]) + dl[v]);
+          for (int v = 0; v < 2; ++v) {
+            const int i = 4 * i4 + 2 * v;
+            f2_unpack(f2_fma(f2_pack(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), c2, v ? l4.y : l4.x), e[2 * v],
+                      e[2 * v + 1]);
+            e[2 * v] = exp2f(e[2 * v]);
+            e[2 * v + 1] = exp2f(e[2 * v + 1]);
+            const f32x2 t = f2_add(f2_pack(__uint_as_float(rp[i]), __uint_as_float(rp[i + 1])), v ? d4.y : d4.x);
+            f2_unpack(f2_mul(f2_pack(e[2 * v], e[2 * v + 1]), t), ds[2 * v], ds[2 * v + 1]);
           }
           pw[2 * i4] = pack_bf16x2(e[0], e[1]);
           pw[2 * i4 + 1] = pack_bf16x2(e[2], e[3]);

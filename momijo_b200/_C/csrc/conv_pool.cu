@@ -226,18 +226,6 @@ struct GatherGeom {
   long long dst_n, dst_m, dst_g;
 };
 
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-
 // taps of one axis that a pixel class meets: t = first + i * step, i < count; source shift = e0 + i * es
 struct AxisTaps {
   int first, step, count, e0, es;
@@ -355,7 +343,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3)
     for (int kk = 0; kk < BK; ++kk) Bs[buf][kk][t] = rb[kk];
   };
 
-  unsigned long long acc[TM][TN / 2];
+  f32x2 acc[TM][TN / 2];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -376,7 +364,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3)
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       float a[TM];
-      unsigned long long b[TN / 2];
+      f32x2 b[TN / 2];
 #pragma unroll
       for (int i = 0; i < TM; i += 4) {
         const float4 v = *reinterpret_cast<const float4*>(&As[buf][kk][ty * TM + i]);
@@ -385,14 +373,14 @@ __global__ void __launch_bounds__(kGatherThreads, 3)
 #pragma unroll
       for (int j = 0; j < TN / 4; ++j) {
         const float4 v = *reinterpret_cast<const float4*>(&Bs[buf][kk][j * (BN * 4 / TN) + tx * 4]);
-        b[2 * j] = pack2(v.x, v.y);
-        b[2 * j + 1] = pack2(v.z, v.w);
+        b[2 * j] = f2_pack(v.x, v.y);
+        b[2 * j + 1] = f2_pack(v.z, v.w);
       }
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
-        const unsigned long long aa = pack2(a[i], a[i]);
+        const f32x2 aa = f2_pack(a[i], a[i]);
 #pragma unroll
-        for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], aa, b[j]);
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = f2_fma(aa, b[j], acc[i][j]);
       }
     }
     if (c + 1 < chunks) stage(buf ^ 1);
@@ -408,7 +396,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3)
     for (int j = 0; j < TN / 2; ++j) {
       const int p = (j >> 1) * (BN * 4 / TN) + tx * 4 + (j & 1) * 2;
       float lo, hi;
-      unpack2(acc[i][j], lo, hi);
+      f2_unpack(acc[i][j], lo, hi);
       if (out_off[p] >= 0) o[out_off[p]] = from_f<T>(lo + bv);
       if (out_off[p + 1] >= 0) o[out_off[p + 1]] = from_f<T>(hi + bv);
     }
@@ -490,7 +478,7 @@ __global__ void __launch_bounds__(kWgThreads, 4)
     for (int i = 0; i < RB; i += 4)
       *reinterpret_cast<float4*>(&Bs[buf][lane][warp * RB + i]) = make_float4(rb[i], rb[i + 1], rb[i + 2], rb[i + 3]);
   };
-  unsigned long long acc[TM][TN / 2];
+  f32x2 acc[TM][TN / 2];
   float sum[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
@@ -523,12 +511,12 @@ __global__ void __launch_bounds__(kWgThreads, 4)
         a[0] = v.x; a[1] = v.y;
       }
       const float4 v = *reinterpret_cast<const float4*>(&Bs[buf][p][tx * 4]);
-      const unsigned long long b0 = pack2(v.x, v.y), b1 = pack2(v.z, v.w);
+      const f32x2 b0 = f2_pack(v.x, v.y), b1 = f2_pack(v.z, v.w);
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
-        const unsigned long long aa = pack2(a[i], a[i]);
-        fma2(acc[i][0], aa, b0);
-        fma2(acc[i][1], aa, b1);
+        const f32x2 aa = f2_pack(a[i], a[i]);
+        acc[i][0] = f2_fma(aa, b0, acc[i][0]);
+        acc[i][1] = f2_fma(aa, b1, acc[i][1]);
       }
     }
     if (c + 1 < chunks) stage(buf ^ 1);
@@ -538,7 +526,7 @@ __global__ void __launch_bounds__(kWgThreads, 4)
 #pragma unroll
         for (int j = 0; j < TN / 2; ++j) {
           float lo, hi;
-          unpack2(acc[i][j], lo, hi);
+          f2_unpack(acc[i][j], lo, hi);
           sum[i][2 * j] += lo;
           sum[i][2 * j + 1] += hi;
           acc[i][j] = 0ull;

@@ -708,33 +708,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 constexpr int kPairBN = 256;
 constexpr int kPairStageBytes = kAStageBytes + (kPairBN / 2) * kGemmBK * 2;  // 32 KiB
 
-// Two fp32 values in one register pair: the f32x2 instructions take half the issue slots of scalar ones and round
-// alike. The fused GELU / GELU' epilogues are bound by issue (25 and 28 instructions an element at 41 % of the
-// issue slots, two or three warps per scheduler), not by a pipe.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(f32x2 v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
+// The fused GELU / GELU' epilogues are bound by issue (25 and 28 instructions an element at 41 % of the issue slots with
+// scalar arithmetic, two or three warps per scheduler), not by a pipe.
 // the two bf16 halves of a word, widened (their bits are the upper halves of the fp32 values)
 __device__ __forceinline__ f32x2 f2_from_bf16(uint32_t u) {
   return f2_pack(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
