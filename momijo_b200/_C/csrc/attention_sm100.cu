@@ -666,10 +666,14 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tmem_ld_wait();
         if (tr && j < 6) trace_stamp(p.trace, blockIdx.x, 8 + 24 * t + 4 * j + 1);
         if (need_mask) {
+          // keys behind the query (causal) and past the end: one bit per column
+          const int n = min(p.T, p.causal ? q_idx + 1 : p.T) - kv0;   // live columns
+          const uint32_t m0 = n >= 32 ? 0xffffffffu : n <= 0 ? 0u : (1u << n) - 1u;
+          const uint32_t m1 = n >= 64 ? 0xffffffffu : n <= 32 ? 0u : (1u << (n - 32)) - 1u;
 #pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const int kv = kv0 + i;
-            if (kv >= p.T || (p.causal && kv > q_idx)) s[i] = 0xff800000u;  // -inf
+          for (int i = 0; i < 32; ++i) {
+            s[i] = (m0 & (1u << i)) ? s[i] : 0xff800000u;  // -inf
+            s[i + 32] = (m1 & (1u << i)) ? s[i + 32] : 0xff800000u;
           }
         }
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
