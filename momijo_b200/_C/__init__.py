@@ -195,23 +195,28 @@ class NativeError(RuntimeError):
 _NVTX = os.environ.get("MOMIJO_NVTX", "0") == "1"
 
 
+_FNS = {}   # name -> (bound function, kernels launched per call)
+
+
 def call(name: str, *args):
     """Call an exported launcher, count its kernels and raise on a non-zero return code. With
     ``MOMIJO_NVTX=1`` every call is wrapped in an NVTX range named after the launcher, so that a
     timeline tool shows which front-end call produced which kernels."""
     global launches
-    fn = getattr(lib(), name)
+    entry = _FNS.get(name)
+    if entry is None:
+        entry = _FNS[name] = (getattr(lib(), name), _SIGS[name][1])
     if _NVTX:
         import torch
 
         torch.cuda.nvtx.range_push(name)
         try:
-            rc = fn(*args)
+            rc = entry[0](*args)
         finally:
             torch.cuda.nvtx.range_pop()
     else:
-        rc = fn(*args)
-    launches += _SIGS[name][1]
+        rc = entry[0](*args)
+    launches += entry[1]
     if rc != 0:
         raise NativeError(f"{name} failed with code {rc}")
     return rc
@@ -274,6 +279,9 @@ def status_tensor(device=None):
     """Per-device int32[4] status word that kernels fill when a bounded wait runs out."""
     import torch
 
+    t = _STATUS.get(device)
+    if t is not None:
+        return t
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     t = _STATUS.get(dev)
     if t is None:

@@ -168,11 +168,14 @@ def _gemm_split_k(a, b, out, accumulate, M, N, K, S, bn, tall=False):
 
 
 def _check_2d(t, name):
-    if t.dim() != 2 or t.stride(1) != 1:
+    """Leading dimension of a bf16 matrix with unit inner stride."""
+    st = t.stride()
+    if len(st) != 2 or st[1] != 1:
         raise ValueError(f"{name} must be 2-D with unit inner stride, got shape {tuple(t.shape)} "
                          f"strides {t.stride()}")
     if t.dtype != torch.bfloat16:
         raise TypeError(f"{name} must be bfloat16, got {t.dtype}")
+    return st[0]
 
 
 def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_f32=False, accumulate=False, bias=None,
@@ -182,22 +185,27 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_f32=False, accumulate=Fa
 
     a: ``[M, K]`` (or ``[K, M]`` when ``a_mn``); b: ``[N, K]`` (or ``[K, N]`` when ``b_mn``).
     """
-    _check_2d(a, "a")
-    _check_2d(b, "b")
-    M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
-    N, Kb = (b.shape[1], b.shape[0]) if b_mn else (b.shape[0], b.shape[1])
+    lda, ldb = _check_2d(a, "a"), _check_2d(b, "b")
+    M, K = a.shape
+    N, Kb = b.shape
+    if a_mn:
+        M, K = K, M
+    if b_mn:
+        N, Kb = Kb, N
     if K != Kb:
         raise ValueError(f"contraction mismatch: {K} vs {Kb}")
     aux = dgelu_aux if dgelu_aux is not None else (add_aux if add_aux is not None else mul_aux)
     if out is None:
-        out = torch.empty((M, N), dtype=torch.float32 if out_f32 else torch.bfloat16, device=a.device)
+        out = a.new_empty((M, N), dtype=torch.float32) if out_f32 else a.new_empty((M, N))
+        ldo = N
         accumulate = False
     else:
         out_f32 = out.dtype == torch.float32
         if out.dim() != 2 or out.shape[0] != M or out.shape[1] != N or out.stride(1) != 1:
             raise ValueError("bad out shape")
+        ldo = out.stride(0)
     if gelu and pre_out is None:
-        pre_out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
+        pre_out = a.new_empty((M, N))
 
     if not a.is_cuda:
         A = (a.t() if a_mn else a).float()
@@ -242,9 +250,8 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_f32=False, accumulate=Fa
         epi |= EPI_ACCUMULATE
     if row_scale is not None:
         epi |= EPI_ROW_SCALE
-    if aux is not None:
-        _check_2d(aux, "aux")
-    if N % 8 != 0 and out.stride(0) % 8 != 0:
+    ldaux = _check_2d(aux, "aux") if aux is not None else 0
+    if N % 8 != 0 and ldo % 8 != 0:
         raise ValueError("output leading dimension must be a multiple of 8 elements")
     if (a_mn and b_mn and epi in (0, EPI_ACCUMULATE) and out.is_contiguous() and (M * N) % 8 == 0
             and M % 8 == 0 and N % 8 == 0):
@@ -260,9 +267,8 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_f32=False, accumulate=Fa
             bn, tall = 256, True
         else:
             bn = pick_bn(M, N)
-    _C.call("mmj_gemm_bf16", _C.ptr(a), a.stride(0), int(a_mn), _C.ptr(b), b.stride(0), int(b_mn),
-            _C.ptr(out), out.stride(0), M, N, K, epi, _C.ptr(bias), _C.ptr(aux),
-            aux.stride(0) if aux is not None else 0, _C.ptr(pre_out),
+    _C.call("mmj_gemm_bf16", a.data_ptr(), lda, int(a_mn), b.data_ptr(), ldb, int(b_mn),
+            out.data_ptr(), ldo, M, N, K, epi, _C.ptr(bias), _C.ptr(aux), ldaux, _C.ptr(pre_out),
             pre_out.stride(0) if pre_out is not None else 0, _C.ptr(row_scale), bn | (TALL if tall else 0),
-            _C.ptr(_C.status_tensor(a.device)), _C.current_stream())
+            _C.status_tensor(a.device).data_ptr(), _C.current_stream())
     return (out, pre_out) if gelu else out
