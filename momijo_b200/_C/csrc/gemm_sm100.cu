@@ -1081,6 +1081,232 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
 }
 
 // ---------------------------------------------------------------------------------------------
+// Split kernel: 128 x 64 tiles whose contraction is cut over a cluster of S CTAs
+// ---------------------------------------------------------------------------------------------
+// For products with few output tiles (a handful of rows through a projection, short prompts). There the time is one
+// CTA's walk along K, about 1000 cycles for each 64-deep block (one SM's share of the L2 plus latency), while most SMs
+// idle: 8 x 2304 x 768 took 14.1 us on 18 CTAs, 113 x 768 x 3072 40 us on 6. Narrow tiles and up to eight ranges of K
+// put the operands' bytes on as many SMs as there are; the partial tiles meet in distributed shared memory, where CTA r
+// of a cluster adds columns [64 r / S, 64 (r + 1) / S) over the ranks in order (the result does not depend on timing)
+// and runs the epilogue on them: 8.3 us and 10.6 us (2 and 8 ranges of K; the rule that picks them is the front end's).
+constexpr int kSplitBN = 64, kSplitStages = 4, kSplitThreads = 192;
+constexpr int kSplitStageBytes = kAStageBytes + kSplitBN * kGemmBK * 2;   // 24 KiB
+constexpr int kSplitPitch = 68;                                          // floats; rows 16-byte aligned, conflict free
+
+// Epilogue of eight consecutive columns of one row.
+__device__ __forceinline__ void epilogue_cols8(const GemmParams& p, float (&v)[8], int row, int col0) {
+  const int epi = p.epi;
+  const bool full = p.vec_ok && col0 + 8 <= p.N;
+  auto load8 = [&](const __nv_bfloat16* src, float (&x)[8]) {
+    if (full) {
+      const uint4 q = *reinterpret_cast<const uint4*>(src);
+      const float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
+      x[0] = f0.x; x[1] = f0.y; x[2] = f1.x; x[3] = f1.y; x[4] = f2.x; x[5] = f2.y; x[6] = f3.x; x[7] = f3.y;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = (col0 + i < p.N) ? __bfloat162float(src[i]) : 0.f;
+    }
+  };
+  auto store8 = [&](__nv_bfloat16* dst, const float (&x)[8]) {
+    if (full) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]),
+                                                  pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (col0 + i < p.N) dst[i] = __float2bfloat16(x[i]);
+    }
+  };
+  float x[8];
+  if (epi & kEpiBias) {
+    load8(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0, x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] += x[i];
+  }
+  if (epi & kEpiGelu) {
+    store8(reinterpret_cast<__nv_bfloat16*>(p.D2) + (long long)row * p.ldd2 + col0, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = gelu_tanh(v[i]);
+  }
+  if (epi & kEpiSilu) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = v[i] / (1.0f + __expf(-v[i]));
+  }
+  if (epi & (kEpiDGelu | kEpiAddAux | kEpiMulAux)) {
+    load8(reinterpret_cast<const __nv_bfloat16*>(p.aux) + (long long)row * p.ldaux + col0, x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      v[i] = (epi & kEpiDGelu) ? v[i] * gelu_tanh_grad(x[i]) : (epi & kEpiMulAux) ? v[i] * x[i] : v[i] + x[i];
+  }
+  if (epi & kEpiRowScale) {
+    const float sc = p.row_scale[row];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] *= sc;
+  }
+  if (epi & kEpiOutF32) {
+    float* d = reinterpret_cast<float*>(p.D) + (long long)row * p.ldd + col0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (col0 + i < p.N) d[i] = (epi & kEpiAccumulate) ? d[i] + v[i] : v[i];
+  } else {
+    __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + (long long)row * p.ldd + col0;
+    if (epi & kEpiAccumulate) {
+      load8(d, x);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] += x[i];
+    }
+    store8(d, v);
+  }
+}
+
+template <int S>
+__global__ void __launch_bounds__(kSplitThreads)
+gemm_bf16_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                       const GemmParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  __shared__ __align__(8) uint64_t full_bar[kSplitStages], empty_bar[kSplitStages], tfull_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = S > 1 ? (int)cluster_ctarank() : 0;
+  const int num_m = (p.M + kGemmBM - 1) / kGemmBM;
+  const int num_k = (p.K + kGemmBK - 1) / kGemmBK;
+  const int tile = (int)blockIdx.x / S;
+  const int n_tile = tile / num_m;
+  const int m0 = (tile - n_tile * num_m) * kGemmBM, n0 = n_tile * kSplitBN;
+  const int kb0 = rank * num_k / S, kb1 = (rank + 1) * num_k / S;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kSplitStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&tfull_bar, 1);
+    abort_flag = 0;
+    mbar_fence_init();
+    prefetch_tmap(&tmA);
+    prefetch_tmap(&tmB);
+  }
+  if (warp == 1) {
+    tmem_alloc(&tmem_slot, kSplitBN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  pdl_wait();  // nothing above touched global memory
+  pdl_trigger();
+
+  uint32_t acc[kSplitBN];
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+        const int s = i % kSplitStages;
+        if (!mbar_wait(&empty_bar[s], ((i / kSplitStages) & 1) ^ 1, &abort_flag, p.status, kTimeoutEmpty, kb)) break;
+        uint8_t* sA = smem + s * kSplitStageBytes;
+        mbar_expect_tx(&full_bar[s], kSplitStageBytes);
+        tma_load_2d(sA, &tmA, &full_bar[s], kb * kGemmBK, m0);
+        if (!p.b_mn) tma_load_2d(sA + kAStageBytes, &tmB, &full_bar[s], kb * kGemmBK, n0);
+        else tma_load_2d(sA + kAStageBytes, &tmB, &full_bar[s], n0, kb * kGemmBK);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    const uint32_t idesc = make_idesc_bf16(kGemmBM, kSplitBN, 0, p.b_mn);
+    const uint32_t b_kstep = (p.b_mn ? 2048u : 32u) >> 4;
+    const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), 16);
+    const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem) + (uint32_t)kAStageBytes, p.b_mn ? 8192u : 16u);
+    for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+      const int s = i % kSplitStages;
+      if (!mbar_wait_warp(&full_bar[s], (i / kSplitStages) & 1, &abort_flag, p.status, kTimeoutFull, kb)) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t a_lo = a_lo0 + s * (kSplitStageBytes >> 4), b_lo = b_lo0 + s * (kSplitStageBytes >> 4);
+#pragma unroll
+        for (int k = 0; k < kGemmBK / 16; ++k)
+          umma_bf16_ss(tmem_base, smem_desc(a_lo + k * 2), smem_desc(b_lo + k * b_kstep), idesc,
+                       (i > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&empty_bar[s]);
+        if (kb + 1 == kb1) umma_commit(&tfull_bar);
+      }
+      __syncwarp();
+    }
+  } else {
+    const int quad = warp & 3;
+    const int row = quad * 32 + lane;
+    ok = mbar_wait_warp(&tfull_bar, 0, &abort_flag, p.status, kTimeoutTmemFull, tile);
+    if (ok) {
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
+      tmem_ld_32x32(t_row, *reinterpret_cast<uint32_t(*)[32]>(&acc[0]));
+      tmem_ld_32x32(t_row + 32, *reinterpret_cast<uint32_t(*)[32]>(&acc[32]));
+      tmem_ld_wait();
+      if (S == 1) {
+        if (m0 + row < p.M) {
+#pragma unroll
+          for (int c = 0; c < kSplitBN; c += 8) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(acc[c + i]);
+            if (n0 + c < p.N) epilogue_cols8(p, v, m0 + row, n0 + c);
+          }
+        }
+      } else {
+        // every product of this CTA has completed: its stages are free for the partial tile
+        float* red = reinterpret_cast<float*>(smem) + row * kSplitPitch;
+#pragma unroll
+        for (int c = 0; c < kSplitBN; c += 4)
+          *reinterpret_cast<float4*>(red + c) = make_float4(__uint_as_float(acc[c]), __uint_as_float(acc[c + 1]),
+                                                             __uint_as_float(acc[c + 2]), __uint_as_float(acc[c + 3]));
+      }
+    }
+  }
+  if (S > 1) {
+    cluster_sync_all();
+    if (warp >= 2) {
+      constexpr int kCols = kSplitBN / S;
+      const int row = (warp & 3) * 32 + lane;
+      const int c0 = rank * kCols;
+      float v[kCols];
+#pragma unroll
+      for (int i = 0; i < kCols; ++i) v[i] = 0.f;
+      const uint32_t mine = smem_u32(smem) + (uint32_t)(row * kSplitPitch + c0) * 4u;
+#pragma unroll
+      for (int r = 0; r < S; ++r) {
+        const uint32_t peer = mapa_shared(mine, (uint32_t)r);
+#pragma unroll
+        for (int i = 0; i < kCols; i += 4) {
+          float4 q;
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w)
+                       : "r"(peer + i * 4u)
+                       : "memory");
+          v[i] += q.x; v[i + 1] += q.y; v[i + 2] += q.z; v[i + 3] += q.w;
+        }
+      }
+      if (ok && m0 + row < p.M) {
+#pragma unroll
+        for (int c = 0; c < kCols; c += 8) {
+          float u[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) u[i] = v[c + i];
+          if (n0 + c0 + c < p.N) epilogue_cols8(p, u, m0 + row, n0 + c0 + c);
+        }
+      }
+    }
+    cluster_sync_all();  // no CTA leaves while a peer may still read its partial tile
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    tmem_dealloc(tmem_base, kSplitBN);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -1248,6 +1474,67 @@ int launch_gemm(GemmParams& p, const void* A, long long lda, long long a_rows, c
   return (int)cudaGetLastError();
 }
 
+// 16-byte vector accesses in the epilogue need aligned bases and leading dimensions.
+static int epilogue_vec_ok(const GemmParams& p) {
+  const int out_elems = (p.epi & kEpiOutF32) ? 4 : 8;
+  bool ok = (p.ldd % out_elems == 0) && (((uintptr_t)p.D & 15) == 0);
+  if (p.epi & kEpiBias) ok = ok && (((uintptr_t)p.bias & 15) == 0);
+  if (p.epi & kEpiGelu) ok = ok && (p.ldd2 % 8 == 0) && (((uintptr_t)p.D2 & 15) == 0);
+  if (p.epi & (kEpiDGelu | kEpiAddAux | kEpiMulAux)) ok = ok && (p.ldaux % 8 == 0) && (((uintptr_t)p.aux & 15) == 0);
+  return ok ? 1 : 0;
+}
+
+// Split kernel launcher: plain products with K-major A. `splits`: 1, 2, 4 or 8 ranges of K.
+int launch_gemm_split(GemmParams& p, const void* A, long long lda, long long a_rows, const void* B, long long ldb,
+                      long long b_rows, int splits, cudaStream_t stream) {
+  if (p.M <= 0 || p.N <= 0) return 0;
+  if ((lda % 8) != 0 || (ldb % 8) != 0) return -2;
+  if (((uintptr_t)A & 15) || ((uintptr_t)B & 15)) return -3;
+  if (p.a_mn || (p.epi & kEpiScatterPeers) || p.K <= 0) return -7;
+  p.vec_ok = epilogue_vec_ok(p);
+  CUtensorMap tmA, tmB;
+  int rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)p.K, (uint64_t)a_rows, (uint64_t)lda, 64, 128);
+  if (rc) return rc;
+  if (!p.b_mn)
+    rc = make_tmap_bf16_2d(&tmB, B, (uint64_t)p.K, (uint64_t)b_rows, (uint64_t)ldb, 64, kSplitBN);
+  else
+    rc = make_tmap_bf16_2d(&tmB, B, (uint64_t)p.N, (uint64_t)b_rows, (uint64_t)ldb, 64, 64);
+  if (rc) return rc;
+  const int smem_bytes = kSplitStages * kSplitStageBytes + 1024;
+  typedef void (*SplitKernel)(CUtensorMap, CUtensorMap, GemmParams);
+  SplitKernel kernel = splits == 1   ? &gemm_bf16_split_kernel<1>
+                       : splits == 2 ? &gemm_bf16_split_kernel<2>
+                       : splits == 4 ? &gemm_bf16_split_kernel<4>
+                       : splits == 8 ? &gemm_bf16_split_kernel<8>
+                                     : nullptr;
+  if (kernel == nullptr) return -4;
+  static bool attr_set = false;
+  if (!attr_set) {
+    for (SplitKernel k : {&gemm_bf16_split_kernel<1>, &gemm_bf16_split_kernel<2>, &gemm_bf16_split_kernel<4>,
+                          &gemm_bf16_split_kernel<8>}) {
+      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+      if (e != cudaSuccess) return (int)e;
+    }
+    attr_set = true;
+  }
+  const long long tiles = (long long)((p.M + kGemmBM - 1) / kGemmBM) * ((p.N + kSplitBN - 1) / kSplitBN);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * splits));
+  cfg.blockDim = dim3(kSplitThreads);
+  cfg.dynamicSmemBytes = (size_t)smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p);
+  return (int)(e != cudaSuccess ? e : cudaGetLastError());
+}
+
 // Pair kernel launcher: plain products only (no flags, groups, gathered or scattered operands).
 static int g_pair_max_dyn = 0;
 static int g_pair_clusters = 0;
@@ -1257,15 +1544,7 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
   if (p.M <= 0 || p.N <= 0) return 0;
   if ((lda % 8) != 0 || (ldb % 8) != 0) return -2;
   if (p.epi & kEpiScatterPeers) return -7;
-  {
-    const int out_elems = (p.epi & kEpiOutF32) ? 4 : 8;
-    bool ok = (p.ldd % out_elems == 0) && (((uintptr_t)p.D & 15) == 0);
-    if (p.epi & kEpiBias) ok = ok && (((uintptr_t)p.bias & 15) == 0);
-    if (p.epi & kEpiGelu) ok = ok && (p.ldd2 % 8 == 0) && (((uintptr_t)p.D2 & 15) == 0);
-    if (p.epi & (kEpiDGelu | kEpiAddAux | kEpiMulAux))
-      ok = ok && (p.ldaux % 8 == 0) && (((uintptr_t)p.aux & 15) == 0);
-    p.vec_ok = ok ? 1 : 0;
-  }
+  p.vec_ok = epilogue_vec_ok(p);
   if (((uintptr_t)A & 15) || ((uintptr_t)B & 15)) return -3;
   p.bn = kPairBN;
   CUtensorMap tmA, tmB;
@@ -1361,6 +1640,8 @@ MMJ_API int mmj_gemm_bf16(const void* A, long long lda, int a_mn, const void* B,
   p.bias = bias; p.aux = aux; p.ldaux = ldaux;
   p.row_scale = row_scale;
   p.status = status;
+  if ((bn >> 14) & 1)  // bit 14 of `bn`: 128 x 64 tiles, K cut into (bn >> 16) ranges over a cluster
+    return launch_gemm_split(p, A, lda, a_mn ? K : M, B, ldb, b_mn ? K : N, bn >> 16, (cudaStream_t)stream);
   if ((bn >> 13) & 1)  // bit 13 of `bn`: CTA-pair kernel, 256 x 256 tiles
     return launch_gemm_pair(p, A, lda, a_mn ? K : M, B, ldb, b_mn ? K : N, (cudaStream_t)stream);
   return launch_gemm(p, A, lda, a_mn ? K : M, B, ldb, b_mn ? K : N, 0, (cudaStream_t)stream);

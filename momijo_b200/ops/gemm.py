@@ -29,6 +29,7 @@ EPI_SCATTER_PEERS = 256
 EPI_ROW_SCALE = 512
 TALL = 1 << 12   # or-ed into the tile width: 256-row tiles (two 128-row MMAs per B stage)
 PAIR = 1 << 13   # or-ed into the tile width: CTA-pair kernel (cta_group::2), 256 x 256 tiles over two SMs
+SPLIT = 1 << 14  # instead of a tile width: 128 x 64 tiles, contraction cut into (value >> 16) ranges over a cluster
 _PAIR = {"mode": os.environ.get("MOMIJO_GEMM_PAIR", "auto")}   # "0" never, "1" whenever eligible, "auto"
 
 
@@ -41,6 +42,21 @@ def _gelu_tanh_grad(x):
     u = k0 * (x + k1 * x ** 3)
     t = torch.tanh(u)
     return 0.5 * (1 + t) + 0.5 * x * (1 - t * t) * k0 * (1 + 3 * k1 * x * x)
+
+
+def pick_split(M: int, N: int, K: int) -> int:
+    """Ranges of K (1, 2, 4 or 8) for the split kernel, 0 where the larger tiles are the better ones. Measured, larger
+    tiles / split, us: 8 x 2304 x 768 9.8 / 8.3 (2 ranges; 4 ranges, 144 CTAs, 12.8: clusters of four no longer fit one
+    round), 113 x 768 x 3072 26.5 / 10.7 (8), 1 x 4096 x 4096 33.9 / 16.5 (2), 700 x 640 x 2000 14.4 / 11.6 (2),
+    64 x 8192 x 4096 34.4 / 25.0 (1). With more tiles than that a second range finds no SM and pairs of CTAs win
+    (1024 x 768 x 768 8.6 / 9.5), with a short contraction there is nothing to cut (64 x 64 x 64 4.3 / 5.9)."""
+    tiles, blocks = -(-M // 128) * -(-N // 64), -(-K // 64)
+    if blocks < 8 or tiles > (148 if M < 256 else 64):
+        return 0
+    s = 1
+    while s < 8 and tiles * s * 2 <= 128 and blocks >= 4 * s:
+        s *= 2
+    return s
 
 
 def pick_bn(M: int, N: int) -> int:
@@ -258,6 +274,10 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_f32=False, accumulate=Fa
         S, sbn, stall = plan_wgrad(M, N, K)
         if S > 1:
             return _gemm_split_k(a, b, out, accumulate, M, N, K, S, sbn, stall)
+    if bn is None and not tall and pair is None and not a_mn:
+        s = pick_split(M, N, K)
+        if s:
+            bn, pair = SPLIT | s << 16, False
     if pair is None:
         pair = bn is None and not tall and pick_pair(M, N, K)
     if pair:

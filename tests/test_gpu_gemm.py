@@ -146,3 +146,31 @@ def test_gemm_split_k_weight_gradient(force, M, N):
         _close(acc, expect)
     finally:
         mod._SPLITK["force"] = old
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 512), (113, 776, 776), (129, 72, 1000), (200, 64, 4096), (64, 8192, 520)])
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+def test_split_kernel_edges(M, N, K, splits):
+    """Ragged rows, columns and K ranges of every cluster size, each epilogue option, against a product in 64 bits:
+    the result's own rounding to bf16 is 2^-9, fp32 results differ by the order of K additions."""
+    from momijo_b200.ops.gemm import SPLIT
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    a, b, bias, aux = r(M, K), r(N, K) * K ** -0.5, r(N), r(M, N)
+    ref = a.double() @ b.double().t()
+    bn = SPLIT | splits << 16
+
+    def close(got, want, tol=2.0 ** -8):
+        assert float((got.double() - want).norm()) <= tol * float(want.norm())
+
+    close(gemm(a, b, bn=bn), ref)
+    close(gemm(a, b.t().contiguous(), b_mn=True, bn=bn, bias=bias), ref + bias.double())
+    close(gemm(a, b, bn=bn, out_f32=True), ref, 4 * 2.0 ** -24 * K ** 0.5)
+    close(gemm(a, b, bn=bn, add_aux=aux), ref + aux.double())
+    out = aux.clone()
+    close(gemm(a, b, bn=bn, out=out, accumulate=True), ref + aux.double())
+    act, pre = gemm(a, b, bn=bn, bias=bias, gelu=True)
+    close(pre, ref + bias.double())
+    close(act, torch.nn.functional.gelu(ref + bias.double(), approximate="tanh"))
+    assert torch.equal(gemm(a, b, bn=bn), gemm(a, b, bn=bn))
