@@ -319,6 +319,16 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tma
         "r"(c0), "r"(c1)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr,
+                                                 int32_t c0, int32_t c1, int32_t c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      :
+      : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr),
+        "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
 // D (256 rows: 128 TMEM lanes in each CTA) (+)= A * B; A rows and B columns are split over the two
 // CTAs' shared memory at equal offsets. Issued by one thread of the pair's rank-0 CTA.
 __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,

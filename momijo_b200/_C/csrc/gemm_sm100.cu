@@ -759,13 +759,32 @@ __device__ __forceinline__ void staged_store_words(uint8_t* st, int lane, const 
 // Epilogue of a full 32-row, 32-column chunk (16384 x 3072 x 768: GELU 86 -> 75 us, GELU' 99 -> 78 us, of which 13 us
 // came from fetching aux four lanes to a row instead of a row per lane; sixteen epilogue warps instead of eight measured
 // 78 and 81) with the options fixed at compile time. kMode: 1 = bf16 result with an
-// optional bias, 2 = bias, pre-activation kept, GELU, 3 = times GELU'(aux). `bias` / `auxq` hold the chunk's 16 words.
+// optional bias, 2 = bias, pre-activation kept, GELU, 3 = times GELU'(aux), 4 = fp32 result. `bias` / `auxq` hold the chunk's 16 words.
 template <int kMode>
 __device__ __forceinline__ void epilogue_chunk_fixed(const GemmParams& p, const uint32_t (&acc)[32], bool has_bias,
                                                      const uint4 (&extra)[4], long long row0, int col0, uint8_t* st,
                                                      int lane) {
   const uint32_t* ew = reinterpret_cast<const uint32_t*>(extra);
   uint32_t w[16];
+  if (kMode == 4) {   // fp32, 16 columns (64 bytes of a row) at a time
+    float* d = reinterpret_cast<float*>(p.D) + row0 * p.ldd + col0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4*>(st + stage_off(lane, i)) =
+            make_uint4(acc[16 * h + 4 * i], acc[16 * h + 4 * i + 1], acc[16 * h + 4 * i + 2], acc[16 * h + 4 * i + 3]);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int rr = 8 * i + (lane >> 2);
+        *reinterpret_cast<uint4*>(d + rr * p.ldd + 16 * h + (lane & 3) * 4) =
+            *reinterpret_cast<const uint4*>(st + stage_off(rr, lane & 3));
+      }
+      __syncwarp();
+    }
+    return;
+  }
   if (kMode == 2) {
     uint32_t act[16];
 #pragma unroll
@@ -792,7 +811,7 @@ __device__ __forceinline__ void epilogue_chunk_fixed(const GemmParams& p, const 
   staged_store_words(st, lane, w, reinterpret_cast<__nv_bfloat16*>(p.D) + row0 * p.ldd + col0, p.ldd);
 }
 
-// kMode 0: every combination of epilogue options; 1 to 3: the fixed ones of epilogue_chunk_fixed.
+// kMode 0: every combination of epilogue options; 1 to 4: the fixed ones of epilogue_chunk_fixed.
 template <int kMode>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -850,21 +869,21 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   if (num_k > 0 || p.groups_k > 0) {
     if (warp == 0) {
       // ======================= TMA producer (both CTAs) =======================
-      if (lane == 0) {
-        const uint32_t full0 = mapa_shared(smem_u32(&full_bar[0]), 0);  // rank 0's barriers
-        int s = 0;
-        uint32_t ph = 0;
-        bool ok = true;
-        for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-          const KRange kr = krange_of(t, per_group, num_k, p);
-          const TileCoord tc = tile_of(kr.tt, num_m, num_n, p);
-          const int m0 = tc.m_tile * 2 * kGemmBM + (int)rank * kGemmBM;
-          const int n0 = tc.n_tile * kPairBN + (int)rank * (kPairBN / 2);
-          for (int kb = 0; kb < kr.nk; ++kb) {
-            if (!mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, p.status, kTimeoutEmpty, kb)) {
-              ok = false;
-              break;
-            }
+      const uint32_t full0 = mapa_shared(smem_u32(&full_bar[0]), 0);  // rank 0's barriers
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int t = pair; t < num_tiles && ok; t += num_pairs) {
+        const KRange kr = krange_of(t, per_group, num_k, p);
+        const TileCoord tc = tile_of(kr.tt, num_m, num_n, p);
+        const int m0 = tc.m_tile * 2 * kGemmBM + (int)rank * kGemmBM;
+        const int n0 = tc.n_tile * kPairBN + (int)rank * (kPairBN / 2);
+        for (int kb = 0; kb < kr.nk; ++kb) {
+          if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, p.status, kTimeoutEmpty, kb)) {
+            ok = false;
+            break;
+          }
+          if (elect_one()) {
             uint8_t* sA = smem + (size_t)s * kPairStageBytes;
             uint8_t* sB = sA + kAStageBytes;
             if (leader) mbar_expect_tx(&full_bar[s], 2u * (uint32_t)kPairStageBytes);
@@ -872,18 +891,23 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
             const int k0 = kr.k_begin + kb * kGemmBK;
             if (!p.a_mn) {
               tma_load_2d_pair(sA, &tmA, fb, k0, m0);
+            } else if (p.a_panels) {
+              tma_load_3d_pair(sA, &tmA, fb, 0, k0, m0 >> 6);
             } else {
               tma_load_2d_pair(sA, &tmA, fb, m0, k0);
               tma_load_2d_pair(sA + 8192, &tmA, fb, m0 + 64, k0);
             }
             if (!p.b_mn) {
               tma_load_2d_pair(sB, &tmB, fb, k0, n0);
+            } else if (p.b_panels) {
+              tma_load_3d_pair(sB, &tmB, fb, 0, k0, n0 >> 6);
             } else {
               tma_load_2d_pair(sB, &tmB, fb, n0, k0);
               tma_load_2d_pair(sB + 8192, &tmB, fb, n0 + 64, k0);
             }
-            if (++s == stages) { s = 0; ph ^= 1; }
           }
+          __syncwarp();
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
       }
     } else if (warp == 1) {
@@ -973,12 +997,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         uint8_t* st = (m0 + quad * 32 + 32 <= p.M) ? epi_stage[warp - 2] : nullptr;
         if (kMode != 0 && st != nullptr && n0 + kPairBN <= p.N) {
           // full tile: the next chunk's accumulator and operand are requested before this chunk is worked on
-          const bool has_bias = kMode != 3 && (p.epi & kEpiBias) != 0;
+          const bool has_bias = kMode <= 2 && (p.epi & kEpiBias) != 0;
           const uint4* ext = kMode == 3
               ? reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.aux) +
                                                (long long)(m0 + quad * 32 + (lane >> 2)) * p.ldaux + n0) + (lane & 3)
               : reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.bias) + n0);
-          const long long row0 = m0 + quad * 32;
+          const long long row0 = m0 + quad * 32 + out_row0;
           constexpr int kStep = kEpiWarps / 4, kChunks = kPairBN / 32 / kStep;
           uint32_t r[2][32];
           uint4 e[2][4];
@@ -1357,6 +1381,7 @@ struct TmapSlot {
   bool used;
 };
 constexpr int kTmapCacheSlots = 1024;
+constexpr uint32_t kPanelBox = 0xffffffffu;   // box_outer of a panel map: {64 columns, rows, panels}, box {64, 64, 2}
 
 int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                       uint64_t row_stride_elems, uint32_t box_inner, uint32_t box_outer) {
@@ -1374,11 +1399,12 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return -1;
   ensure_context();
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {row_stride_elems * 2};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
+  const bool panels = box_outer == kPanelBox;
+  cuuint64_t dims[3] = {panels ? 64 : inner, outer, panels ? inner / 64 : 1};
+  cuuint64_t strides[2] = {row_stride_elems * 2, 128};
+  cuuint32_t box[3] = {box_inner, panels ? 64u : box_outer, 2};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, panels ? 3 : 2, const_cast<void*>(base), dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return (int)r;
@@ -1386,6 +1412,11 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64
   slot.map = *out;
   slot.used = true;
   return 0;
+}
+
+static int make_tmap_bf16_panels(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
+                                 uint64_t row_stride_elems) {
+  return make_tmap_bf16_2d(out, base, inner, outer, row_stride_elems, 64, kPanelBox);
 }
 
 static int g_sm_count = 0;
@@ -1549,13 +1580,21 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
   p.bn = kPairBN;
   CUtensorMap tmA, tmB;
   int rc;
+  // An MN-major operand whose width is a multiple of 64 is described as panels of 64 columns, so that one load brings
+  // the two panels of a stage; other widths take a load for each (a panel map would run past the last row's end).
+  p.a_panels = p.a_mn && p.M % 64 == 0;
+  p.b_panels = p.b_mn && p.N % 64 == 0;
   if (!p.a_mn)
     rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)p.K, (uint64_t)a_rows, (uint64_t)lda, 64, 128);
+  else if (p.a_panels)
+    rc = make_tmap_bf16_panels(&tmA, A, (uint64_t)p.M, (uint64_t)a_rows, (uint64_t)lda);
   else
     rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)p.M, (uint64_t)a_rows, (uint64_t)lda, 64, 64);
   if (rc) return rc;
   if (!p.b_mn)
     rc = make_tmap_bf16_2d(&tmB, B, (uint64_t)p.K, (uint64_t)b_rows, (uint64_t)ldb, 64, kPairBN / 2);
+  else if (p.b_panels)
+    rc = make_tmap_bf16_panels(&tmB, B, (uint64_t)p.N, (uint64_t)b_rows, (uint64_t)ldb);
   else
     rc = make_tmap_bf16_2d(&tmB, B, (uint64_t)p.N, (uint64_t)b_rows, (uint64_t)ldb, 64, 64);
   if (rc) return rc;
@@ -1571,7 +1610,7 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
     if (e != cudaSuccess) return (int)e;
     const int max_dyn = 232448 - (int)fa.sharedSizeBytes;
     for (PairKernel k : {&gemm_bf16_pair_kernel<0>, &gemm_bf16_pair_kernel<1>, &gemm_bf16_pair_kernel<2>,
-                         &gemm_bf16_pair_kernel<3>}) {
+                         &gemm_bf16_pair_kernel<3>, &gemm_bf16_pair_kernel<4>}) {
       e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
       if (e != cudaSuccess) return (int)e;
     }
@@ -1607,6 +1646,8 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
       else if ((p.epi & ~kEpiBias) == kEpiGelu) kernel = &gemm_bf16_pair_kernel<2>;
       else if (p.epi == kEpiDGelu) kernel = &gemm_bf16_pair_kernel<3>;
     }
+    // the slabs of a split weight gradient: one tile to a CTA, so that nothing hides its epilogue
+    if (p.vec_ok && p.epi == kEpiOutF32) kernel = &gemm_bf16_pair_kernel<4>;
     cudaError_t e = launch_pdl(kernel, dim3(2 * pairs), dim3(kThreads), (size_t)smem_bytes, stream, tmA, tmB, p);
     if (e != cudaSuccess) return (int)e;
   }

@@ -26,6 +26,7 @@ enum GemmEpi : int {
 struct GemmParams {
   int M, N, K;
   int a_mn, b_mn;  // 0: operand is K-major ([rows, K]); 1: MN-major ([K, rows])
+  int a_panels, b_panels;  // pair kernel: the MN-major operand's map has 64-column panels as its third dimension
   int bn;          // N tile: 64, 128 or 256
   int bm2;         // 1: tiles are 256 rows tall (two 128-row MMAs share every B stage)
   int comm_rot;    // first gather granule the communication CTAs visit (granule units)
