@@ -382,10 +382,20 @@ __global__ void colsum_finalize_kernel(const float* __restrict__ scratch,
 }
 
 // ---- split-K reduction: out[i] (+)= sum_s parts[s][i]  (fp32 slabs -> bf16) ---------------------
+// With `bias_part` [S, M] it adds up a bias gradient's parts as well (bf16 or fp32 output).
 __global__ void splitk_reduce_kernel(const float* __restrict__ parts, long long slab, int S,
-                                     __nv_bfloat16* __restrict__ out, long long n, int accumulate) {
+                                     __nv_bfloat16* __restrict__ out, long long n, int accumulate,
+                                     const float* __restrict__ bias_part, int M, __nv_bfloat16* __restrict__ db,
+                                     float* __restrict__ db32, int db_accumulate) {
   pdl_wait();
   pdl_trigger();
+  if (bias_part != nullptr)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
+      float v = 0.f;
+      for (int s = 0; s < S; ++s) v += bias_part[(long long)s * M + i];
+      if (db32 != nullptr) db32[i] = db_accumulate ? db32[i] + v : v;
+      else db[i] = __float2bfloat16(db_accumulate ? __bfloat162float(db[i]) + v : v);
+    }
   for (long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 8; i < n;
        i += (long long)gridDim.x * blockDim.x * 8) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -707,7 +717,16 @@ MMJ_API int mmj_splitk_reduce(const float* parts, long long slab, int S, void* o
   if (n == 0) return 0;
   if (n % 8 || slab % 4 || S < 1) return -1;
   launch_pdl(splitk_reduce_kernel, dim3(grid_for(n / 8, 256)), dim3(256), 0, STREAM, parts, slab, S,
-             (__nv_bfloat16*)out, n, accumulate);
+             (__nv_bfloat16*)out, n, accumulate, (const float*)nullptr, 0, (__nv_bfloat16*)nullptr, (float*)nullptr, 0);
+  return (int)cudaGetLastError();
+}
+// out[i] (+)= sum of S slabs, and db[m] (+)= sum of S rows of bias_part; db bf16, or db32 fp32 where that is given.
+MMJ_API int mmj_wgrad_fold(const float* parts, long long slab, int S, void* out, long long n, int accumulate,
+                           const float* bias_part, int M, void* db, float* db32, int db_accumulate, void* stream) {
+  if (n % 8) return -1;
+  if (n == 0) return 0;
+  launch_pdl(splitk_reduce_kernel, dim3(grid_for(n / 8, 256)), dim3(256), 0, STREAM, parts, slab, S,
+             (__nv_bfloat16*)out, n, accumulate, bias_part, M, (__nv_bfloat16*)db, db32, db_accumulate);
   return (int)cudaGetLastError();
 }
 

@@ -811,7 +811,11 @@ __device__ __forceinline__ void epilogue_chunk_fixed(const GemmParams& p, const 
   staged_store_words(st, lane, w, reinterpret_cast<__nv_bfloat16*>(p.D) + row0 * p.ldd + col0, p.ldd);
 }
 
-// kMode 0: every combination of epilogue options; 1 to 4: the fixed ones of epilogue_chunk_fixed.
+// kMode 0: every combination of epilogue options; 1 to 4: the fixed ones of epilogue_chunk_fixed; 5: as 4, and the column
+// sums of A (an MN-major dy: the bias gradient of the layer whose weight gradient this is) into p.bias_part. The epilogue
+// warps are idle during a split product's one main loop: those of the CTAs with the first column tile add up their A
+// stages once the products have read them, and every CTA's stages return through its epilogue warps. The four column
+// sums of a GPT-2 layer (19 + 15 + 8 + 8 us and a 3 us fold each) re-read the same dy from HBM.
 template <int kMode>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -820,6 +824,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   __shared__ __align__(8) uint64_t full_bar[kGemmMaxStages];
   __shared__ __align__(8) uint64_t empty_bar[kGemmMaxStages];
+  __shared__ __align__(8) uint64_t done_bar[kGemmMaxStages];   // kMode 5: the stage's products have read it
   __shared__ __align__(8) uint64_t tfull_bar[2];
   __shared__ __align__(8) uint64_t tempty_bar[2];
   __shared__ uint32_t tmem_slot;
@@ -837,7 +842,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+      mbar_init(&empty_bar[s], kMode == 5 ? kEpiWarps : 1);
+      if (kMode == 5) mbar_init(&done_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
@@ -950,7 +956,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
                 umma_bf16_ss_pair(d_tmem, smem_desc(a_lo + k * a_kstep), smem_desc(b_lo + k * b_kstep), idesc,
                                   (kb > 0 || k > 0) ? 1u : 0u);
               // the stage is free in both CTAs once these MMAs retire
-              umma_commit_pair_both(&empty_bar[s]);
+              umma_commit_pair_both(kMode == 5 ? &done_bar[s] : &empty_bar[s]);
               if (kb + 1 == kr.nk) umma_commit_pair_both(&tfull_bar[acc]);
             }
             __syncwarp();
@@ -966,12 +972,55 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       const uint32_t tempty0 = mapa_shared(smem_u32(&tempty_bar[0]), 0);
       int acc = 0;
       uint32_t acc_ph = 0;
+      int cs = 0;          // kMode 5: the stage whose columns come next
+      uint32_t cph = 0;
       for (int t = pair; t < num_tiles; t += num_pairs) {
         const KRange kr = krange_of(t, per_group, num_k, p);
         const TileCoord tc = tile_of(kr.tt, num_m, num_n, p);
         const int m0 = tc.m_tile * 2 * kGemmBM + (int)rank * kGemmBM;
         const int n0 = tc.n_tile * kPairBN;
         const int out_row0 = kr.g * p.M;  // grouped-K: group g writes rows [g*M, (g+1)*M)
+        if (kMode == 5) {
+          // warp: one 64-column panel of A, 16 of the stage's 64 rows; lane: two columns
+          const int panel = (warp - 2) & 1, r0 = ((warp - 2) >> 1) * 16;
+          f32x2 total = 0ull, part = 0ull;   // short chains: eight stages, then into the total
+          bool ok = true;
+          for (int kb = 0; kb < kr.nk; ++kb) {
+            if (!mbar_wait_warp(&done_bar[cs], cph, &abort_flag, p.status, kTimeoutFull, kb)) { ok = false; break; }
+            if (tc.n_tile == 0) {
+              const uint8_t* base = smem + (size_t)cs * kPairStageBytes + panel * 8192;
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const int rr = r0 + i;   // 128-byte rows, 16-byte pieces XORed with the row's low bits
+                part = f2_add(part, f2_from_bf16(*reinterpret_cast<const uint32_t*>(
+                                        base + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4)));
+              }
+              if ((kb & 7) == 7) {
+                total = f2_add(total, part);
+                part = 0ull;
+              }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty_bar[cs]);
+            if (++cs == stages) { cs = 0; cph ^= 1; }
+          }
+          if (tc.n_tile == 0) {   // (after a timeout too: every epilogue warp meets at the barriers)
+            total = f2_add(total, part);
+            float* mine = reinterpret_cast<float*>(epi_stage[warp - 2]);
+            f2_unpack(total, mine[2 * lane], mine[2 * lane + 1]);
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            const int c = (int)threadIdx.x - 64;
+            if (c < 128 && m0 + c < p.M) {
+              float v = 0.f;
+#pragma unroll
+              for (int q = 0; q < kEpiWarps / 2; ++q)
+                v += reinterpret_cast<const float*>(epi_stage[(c >> 6) + 2 * q])[c & 63];
+              p.bias_part[(long long)kr.g * p.M + m0 + c] = v;
+            }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+          }
+          if (!ok) break;
+        }
         if (kr.nk == 0) {
           const int zrow = m0 + quad * 32 + lane;
           if (zrow < p.M) {
@@ -1044,7 +1093,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
               __syncwarp();
               if (lane == 0) mbar_arrive_cluster(tempty0 + (uint32_t)(acc * sizeof(uint64_t)));
             }
-            epilogue_chunk_fixed<kMode>(p, r[j & 1], has_bias, q, row0, n0 + c * 32, st, lane);
+            epilogue_chunk_fixed<kMode == 5 ? 4 : kMode>(p, r[j & 1], has_bias, q, row0, n0 + c * 32, st, lane);
           }
           if (++acc == 2) { acc = 0; acc_ph ^= 1; }
           continue;
@@ -1606,11 +1655,11 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
   if (g_pair_max_dyn == 0) {
     cudaFuncAttributes fa;
     typedef void (*PairKernel)(CUtensorMap, CUtensorMap, GemmParams);
-    cudaError_t e = cudaFuncGetAttributes(&fa, gemm_bf16_pair_kernel<0>);
+    cudaError_t e = cudaFuncGetAttributes(&fa, gemm_bf16_pair_kernel<5>);
     if (e != cudaSuccess) return (int)e;
     const int max_dyn = 232448 - (int)fa.sharedSizeBytes;
     for (PairKernel k : {&gemm_bf16_pair_kernel<0>, &gemm_bf16_pair_kernel<1>, &gemm_bf16_pair_kernel<2>,
-                         &gemm_bf16_pair_kernel<3>, &gemm_bf16_pair_kernel<4>}) {
+                         &gemm_bf16_pair_kernel<3>, &gemm_bf16_pair_kernel<4>, &gemm_bf16_pair_kernel<5>}) {
       e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
       if (e != cudaSuccess) return (int)e;
     }
@@ -1648,6 +1697,10 @@ int launch_gemm_pair(GemmParams& p, const void* A, long long lda, long long a_ro
     }
     // the slabs of a split weight gradient: one tile to a CTA, so that nothing hides its epilogue
     if (p.vec_ok && p.epi == kEpiOutF32) kernel = &gemm_bf16_pair_kernel<4>;
+    if (p.bias_part != nullptr) {
+      if (!p.vec_ok || !p.a_panels || p.epi != kEpiOutF32) return -8;
+      kernel = &gemm_bf16_pair_kernel<5>;
+    }
     cudaError_t e = launch_pdl(kernel, dim3(2 * pairs), dim3(kThreads), (size_t)smem_bytes, stream, tmA, tmB, p);
     if (e != cudaSuccess) return (int)e;
   }
@@ -1811,6 +1864,22 @@ MMJ_API int mmj_gemm_bf16_reduce_scatter(const void* A, long long lda, const voi
 //   D[g][M, N] = sum over rows k in [group_k[2g], group_k[2g+1]) of A[k, :M]^T B[k, :N]
 // with A: [rows, M] and B: [rows, N] row-major (both MN-major operands; rows outside every range
 // are never read, rows inside a range that hold no token must be zero). D is [groups, M, N].
+// Weight gradient cut into `splits` ranges of the contraction, on CTA pairs: fp32 slabs [splits, M, N] of dy^T x and the
+// column sums of dy [splits, M]. dy: [rows, M] (M % 64 == 0), x: [rows, N]; mmj_wgrad_fold adds both up.
+MMJ_API int mmj_wgrad_bias(const void* dy, long long lddy, const void* x, long long ldx, float* slabs, float* bias_part,
+                           int rows, int M, int N, int splits, const int* ranges_dev, int* status, void* stream) {
+  GemmParams p = {};
+  p.M = M; p.N = N; p.K = rows;
+  p.a_mn = 1; p.b_mn = 1;
+  p.epi = kEpiOutF32;
+  p.D = slabs; p.ldd = N;
+  p.bias_part = bias_part;
+  p.status = status;
+  p.groups_k = splits;
+  p.group_k = ranges_dev;
+  return launch_gemm_pair(p, dy, lddy, rows, x, ldx, rows, (cudaStream_t)stream);
+}
+
 MMJ_API int mmj_gemm_bf16_grouped_k(const void* A, long long lda, const void* B, long long ldb,
                                     void* D, long long ldd, int rows, int M, int N, int groups,
                                     const int* group_k_dev, int out_f32, int accumulate, int bn,

@@ -41,6 +41,7 @@ struct GemmParams {
   const void* aux;
   long long ldaux;
   const float* row_scale;
+  float* bias_part;  // pair kernel, split weight gradients: column sums of A, [groups_k, M]
   int* status;
 
   // Grouped GEMM (MoE experts). tile_group[m_tile] gives the group of each 128-row tile;

@@ -17,7 +17,7 @@ import torch.nn.functional as tF
 from torch.autograd import forward_ad
 
 from .. import _C
-from .gemm import gemm, _gelu_tanh, _gelu_tanh_grad
+from .gemm import gemm, wgrad_bias, _gelu_tanh, _gelu_tanh_grad
 
 bf16 = torch.bfloat16
 
@@ -102,6 +102,18 @@ def _weight_grad(w, dy2d, x2d):
     return gemm(dy2d, x2d, a_mn=True, b_mn=True)
 
 
+def _weight_bias_grad(w, b, dy2d, x2d):
+    """Both parameter gradients of a linear layer; one product makes both where the weight gradient is a split one."""
+    wbuf, wacc = _wgrad_target(w)
+    bbuf, bacc = _wgrad_target(b)
+    dw = wbuf if wbuf is not None else dy2d.new_empty((dy2d.shape[1], x2d.shape[1]))
+    db = bbuf if bbuf is not None else dy2d.new_empty(dy2d.shape[1])
+    if not wgrad_bias(dy2d, x2d, dw, wacc, db, bacc):
+        gemm(dy2d, x2d, a_mn=True, b_mn=True, out=dw, accumulate=wacc)
+        _colsum(dy2d, out=db, accumulate=bacc)
+    return None if wbuf is not None else dw, None if bbuf is not None else db
+
+
 # --------------------------------------------------------------------------------------------
 # linear / MLP
 # --------------------------------------------------------------------------------------------
@@ -132,8 +144,12 @@ class _Linear(torch.autograd.Function):
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dx = gemm(dy2, w, b_mn=True).view(ctx.xshape) if ctx.needs_input_grad[0] else None
-        dw = _weight_grad(ctx.w_ref, dy2, x2) if ctx.needs_input_grad[1] else None
-        db = _bias_grad(ctx.b, dy2) if (ctx.b is not None and ctx.needs_input_grad[2]) else None
+        need_b = ctx.b is not None and ctx.needs_input_grad[2]
+        if need_b and ctx.needs_input_grad[1]:
+            dw, db = _weight_bias_grad(ctx.w_ref, ctx.b, dy2, x2)
+        else:
+            dw = _weight_grad(ctx.w_ref, dy2, x2) if ctx.needs_input_grad[1] else None
+            db = _bias_grad(ctx.b, dy2) if need_b else None
         dres = dy if ctx.has_res else None
         return dx, dw, db, dres
 
@@ -168,11 +184,9 @@ class _MlpGelu(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        dw2 = _weight_grad(rw2, dy2, act)
-        db2 = _bias_grad(rb2, dy2)
+        dw2, db2 = _weight_bias_grad(rw2, rb2, dy2, act) if rb2 is not None else (_weight_grad(rw2, dy2, act), None)
         dpre = gemm(dy2, w2, b_mn=True, dgelu_aux=pre)  # (dy @ W2) * gelu'(pre)
-        dw1 = _weight_grad(rw1, dpre, x2)
-        db1 = _bias_grad(rb1, dpre)
+        dw1, db1 = _weight_bias_grad(rw1, rb1, dpre, x2) if rb1 is not None else (_weight_grad(rw1, dpre, x2), None)
         dx = gemm(dpre, w1, b_mn=True).view(ctx.xshape)
         return dx, dw1, db1, dw2, db2, (dy if ctx.has_res else None)
 

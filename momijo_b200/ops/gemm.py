@@ -167,13 +167,39 @@ def _split_ranges(K: int, S: int, device):
     return r
 
 
+def _slabs(need, device):
+    sc = _SPLITK["scratch"]
+    if sc is None or sc.numel() < need or sc.device != device:
+        sc = torch.empty(need, dtype=torch.float32, device=device)
+        _SPLITK["scratch"] = sc
+    return sc
+
+
+def wgrad_bias(dy, x, out, accumulate, db, db_accumulate) -> bool:
+    """``out (+)= dy^T x`` and ``db (+)= column sums of dy`` in one product where the weight gradient is split over CTA
+    pairs; False (and nothing done) where it is not."""
+    K, M = dy.shape
+    N = x.shape[1]
+    if (not dy.is_cuda or out.dtype != torch.bfloat16 or not out.is_contiguous() or not db.is_contiguous()
+            or M % 64 or N % 8):
+        return False
+    S, _, tall = plan_wgrad(M, N, K)
+    if S <= 1 or tall != "pair":
+        return False
+    lddy, ldx = _check_2d(dy, "a"), _check_2d(x, "b")
+    sc = _slabs(S * M * N, dy.device)
+    part = dy.new_empty(S * M, dtype=torch.float32)
+    _C.call("mmj_wgrad_bias", dy.data_ptr(), lddy, x.data_ptr(), ldx, sc.data_ptr(), part.data_ptr(), K, M, N, S,
+            _C.ptr(_split_ranges(K, S, dy.device)), _C.status_tensor(dy.device).data_ptr(), _C.current_stream())
+    f32 = db.dtype == torch.float32
+    _C.call("mmj_wgrad_fold", sc.data_ptr(), M * N, S, out.data_ptr(), M * N, int(accumulate), part.data_ptr(), M,
+            None if f32 else db.data_ptr(), db.data_ptr() if f32 else None, int(db_accumulate), _C.current_stream())
+    return True
+
+
 def _gemm_split_k(a, b, out, accumulate, M, N, K, S, bn, tall=False):
     """a: [K, M], b: [K, N] (both MN-major). Partial products as fp32 slabs, then one reduction pass."""
-    need = S * M * N
-    sc = _SPLITK["scratch"]
-    if sc is None or sc.numel() < need or sc.device != a.device:
-        sc = torch.empty(need, dtype=torch.float32, device=a.device)
-        _SPLITK["scratch"] = sc
+    sc = _slabs(S * M * N, a.device)
     _C.call("mmj_gemm_bf16_grouped_k", _C.ptr(a), a.stride(0), _C.ptr(b), b.stride(0), _C.ptr(sc), N, K, M, N, S,
             _C.ptr(_split_ranges(K, S, a.device)), 1, 0,
             bn | (PAIR if tall == "pair" else TALL if tall else 0),

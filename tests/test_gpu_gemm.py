@@ -174,3 +174,24 @@ def test_split_kernel_edges(M, N, K, splits):
     close(pre, ref + bias.double())
     close(act, torch.nn.functional.gelu(ref + bias.double(), approximate="tanh"))
     assert torch.equal(gemm(a, b, bn=bn), gemm(a, b, bn=bn))
+
+
+@pytest.mark.parametrize("M,N,K", [(768, 768, 16384), (320, 520, 4100), (2304, 768, 8192), (64, 64, 4096), (768, 768, 100)])
+@pytest.mark.parametrize("db_dtype,acc", [(torch.bfloat16, False), (torch.float32, True)])
+def test_weight_and_bias_gradient_together(M, N, K, db_dtype, acc):
+    """Column sums taken from the stages of a split weight gradient (tails of the last tile and of K among the shapes)
+    and from the separate pass where it is not split."""
+    from momijo_b200.ops import functional as fn
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    dy, x = r(K, M), r(K, N)
+    w, b = torch.nn.Parameter(r(M, N)), torch.nn.Parameter(r(M))
+    w0, b0 = r(M, N), r(M).to(db_dtype)
+    w.main_grad, b.main_grad, w._mg_fresh, b._mg_fresh = w0.clone(), b0.clone(), not acc, not acc
+    assert fn._weight_bias_grad(w, b, dy, x) == (None, None)
+    want_w = dy.double().t() @ x.double() + (w0.double() if acc else 0)
+    want_b = dy.double().sum(0) + (b0.double() if acc else 0)
+    assert float((w.main_grad.double() - want_w).norm()) <= 2.0 ** -8 * float(want_w.norm())
+    tol = 2.0 ** -8 if db_dtype == torch.bfloat16 else 4 * 2.0 ** -24 * K ** 0.5
+    assert float((b.main_grad.double() - want_b).norm()) <= tol * float(want_b.norm())
