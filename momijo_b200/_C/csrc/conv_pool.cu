@@ -29,29 +29,66 @@ template <> __device__ __forceinline__ float from_f<float>(float v) { return v; 
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16(v); }
 
 // ---- im2col: cols[(n, oh, ow), c * kH * kW + kh * kW + kw], row pitch ldc >= C*kH*kW (pad columns = 0) ----
+// A warp owns 32 output positions and 64 columns: it gathers with the positions along its lanes (contiguous in the image
+// rows, one tap for the whole warp, stepped without divisions), turns the tile through shared memory and stores rows of
+// 64 columns. One element per thread, consecutive threads along a row of cols, took two 64-bit divisions each and
+// gathered 32 sectors with every load: 504 us for 100352 x 576 bf16, 82 now.
 template <typename T>
-__global__ void im2col_kernel(const T* __restrict__ x, T* __restrict__ cols, ConvGeom g, long long ldc) {
-  const long long K = (long long)g.C * g.kH * g.kW;
+__global__ void __launch_bounds__(128) im2col_kernel(const T* __restrict__ x, T* __restrict__ cols, ConvGeom g,
+                                                     long long ldc, int vec) {
+  constexpr int V = 16 / sizeof(T);             // elements per 16-byte store
+  constexpr int kPitch = 64 + V;                // rows stay 16-byte aligned
+  __shared__ __align__(16) T tile[4][32 * kPitch];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  T* st = tile[warp];
   const long long rows = (long long)g.N * g.OH * g.OW;
-  const long long total = rows * ldc;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / ldc;
-    const long long k = i - r * ldc;
-    T v = from_f<T>(0.f);
-    if (k < K) {
-      const int kw = (int)(k % g.kW);
-      const int kh = (int)((k / g.kW) % g.kH);
-      const int c = (int)(k / ((long long)g.kW * g.kH));
+  const int K = g.C * g.kH * g.kW;
+  const int k_tiles = (int)((ldc + 63) / 64);
+  const long long units = (rows + 31) / 32 * k_tiles;
+  for (long long u = blockIdx.x * 4LL + warp; u < units; u += gridDim.x * 4LL) {
+    const long long r0 = u / k_tiles * 32;
+    const int k0 = (int)(u % k_tiles) * 64;
+    const long long r = r0 + lane;
+    int h0 = -(1 << 29), w0 = 0;                // a position past the end reads nothing
+    const T* xp = x;
+    if (r < rows) {
       const int ow = (int)(r % g.OW);
-      const int oh = (int)((r / g.OW) % g.OH);
-      const int n = (int)(r / ((long long)g.OW * g.OH));
-      const int h = oh * g.sh - g.ph + kh * g.dh;
-      const int w = ow * g.sw - g.pw + kw * g.dw;
-      if (h >= 0 && h < g.H && w >= 0 && w < g.W)
-        v = x[(((long long)n * g.C + c) * g.H + h) * g.W + w];
+      const long long q = r / g.OW;
+      const int oh = (int)(q % g.OH);
+      h0 = oh * g.sh - g.ph;
+      w0 = ow * g.sw - g.pw;
+      xp = x + (q / g.OH) * g.C * g.H * g.W + (long long)h0 * g.W + w0;
     }
-    cols[i] = v;
+    int c = k0 / (g.kH * g.kW), t = k0 - c * g.kH * g.kW;
+    int kh = t / g.kW, kw = t - kh * g.kW;
+#pragma unroll 8
+    for (int j = 0; j < 64; ++j) {
+      const int dh = kh * g.dh, dw = kw * g.dw;
+      T v = from_f<T>(0.f);
+      if (k0 + j < K && (unsigned)(h0 + dh) < (unsigned)g.H && (unsigned)(w0 + dw) < (unsigned)g.W)
+        v = xp[(long long)c * g.H * g.W + dh * g.W + dw];
+      st[lane * kPitch + j] = v;
+      if (++kw == g.kW) {
+        kw = 0;
+        if (++kh == g.kH) { kh = 0; ++c; }
+      }
+    }
+    __syncwarp();
+    const int n = (int)(ldc - k0 < 64 ? ldc - k0 : 64);
+    if (vec) {
+      constexpr int kLanes = 64 / V;            // lanes per row
+      for (int i = lane; i < 32 * kLanes; i += 32) {
+        const int rr = i / kLanes, cc = (i % kLanes) * V;
+        if (r0 + rr < rows && cc < n)
+          *reinterpret_cast<uint4*>(cols + (r0 + rr) * ldc + k0 + cc) = *reinterpret_cast<const uint4*>(st + rr * kPitch + cc);
+      }
+    } else {
+      for (int i = lane; i < 32 * 64; i += 32) {
+        const int rr = i >> 6, cc = i & 63;
+        if (r0 + rr < rows && cc < n) cols[(r0 + rr) * ldc + k0 + cc] = st[rr * kPitch + cc];
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -729,11 +766,15 @@ using namespace mmj;
 // geom: host int[16] = N, C, H, W, OC, kH, kW, OH, OW, sh, sw, ph, pw, dh, dw, groups. dtype: 0 bf16, 1 fp32.
 MMJ_API int mmj_im2col(const void* x, void* cols, const int* geom, long long ldc, int dtype, void* stream) {
   const ConvGeom g = make_geom(geom);
-  if (!geom_ok(g) || ldc < (long long)g.C * g.kH * g.kW) return -2;
-  const long long total = (long long)g.N * g.OH * g.OW * ldc;
-  DISPATCH(dtype, (im2col_kernel<float><<<grid_1d(total), 256, 0, STREAM>>>((const float*)x, (float*)cols, g, ldc)),
-           (im2col_kernel<__nv_bfloat16><<<grid_1d(total), 256, 0, STREAM>>>((const __nv_bfloat16*)x,
-                                                                              (__nv_bfloat16*)cols, g, ldc)));
+  if (!geom_ok(g) || ldc < (long long)g.C * g.kH * g.kW || ldc > 0x7fffffc0LL) return -2;
+  const long long units = ((long long)g.N * g.OH * g.OW + 31) / 32 * ((ldc + 63) / 64);
+  const long long blocks = (units + 3) / 4;
+  const unsigned grid = (unsigned)(blocks < 148 * 32 ? blocks : 148 * 32);
+  // 16-byte stores need rows that are whole vectors
+  const int vec = ldc % (dtype == 1 ? 4 : 8) == 0 && ((uintptr_t)cols & 15) == 0;
+  DISPATCH(dtype, (im2col_kernel<float><<<grid, 128, 0, STREAM>>>((const float*)x, (float*)cols, g, ldc, vec)),
+           (im2col_kernel<__nv_bfloat16><<<grid, 128, 0, STREAM>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)cols, g, ldc,
+                                                                   vec)));
   return (int)cudaGetLastError();
 }
 MMJ_API int mmj_col2im(const void* cols, void* dx, const int* geom, long long ldc, int dtype, void* stream) {

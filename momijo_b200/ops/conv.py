@@ -78,6 +78,12 @@ def col2im(cols, x_shape, kernel, stride=(1, 1), pad=(0, 0), dilation=(1, 1)):
 
 
 # ---- convolution ----------------------------------------------------------------------------------------
+# bf16 input gradients up to this many filters come from the direct kernel, whose time grows with them, and above from a
+# product and its overlapping sums. Direct / product and sums, us, k3: N32 C64 56x56 16 filters 83 / 282, 32 143 / 290,
+# N32 C128 28x28 48 103 / 155; at 64 filters it depends on the shape (265 / 303, N8 C32 30x30 k5 135 / 85), at 128 511 / 333.
+_DIRECT_DX_CHANNELS = 48
+
+
 def _weight_grad(x, dy, w, geom):
     dw = torch.empty_like(w)
     n = _C.lib().mmj_conv2d_dw_scratch(geom)
@@ -141,8 +147,13 @@ class _Conv2d(torch.autograd.Function):
             if Kp != K:
                 w2 = tF.pad(w2, (0, Kp - K))
             if ctx.needs_input_grad[0]:
-                dcols = gemm(dy2, w2.contiguous(), b_mn=True)              # [N*OH*OW, Kp]
-                dx = col2im(dcols, (N, C, H, W), (kH, kW), stride, pad, dil)
+                if OC <= _DIRECT_DX_CHANNELS:
+                    dx = torch.empty_like(x)
+                    _C.call("mmj_conv2d_dx", _C.ptr(dy), _C.ptr(w), None, _C.ptr(dx), ctx.geom, _dt(x),
+                            _C.current_stream())
+                else:
+                    dcols = gemm(dy2, w2.contiguous(), b_mn=True)              # [N*OH*OW, Kp]
+                    dx = col2im(dcols, (N, C, H, W), (kH, kW), stride, pad, dil)
             if ctx.needs_input_grad[1]:
                 dw2 = gemm(dy2, cols, a_mn=True, b_mn=True)                # [OC, Kp]
                 dw = dw2[:, :K].reshape(OC, C, kH, kW).contiguous()

@@ -131,3 +131,29 @@ def test_conv2d_tile_edges_against_64_bits(N, C, H, W, OC, k, s, p, d, g):
     terms = [C // g * kh * kw, OC // g * kh * kw, N * y.shape[2] * y.shape[3], N * y.shape[2] * y.shape[3]]
     for a, e, n in zip(got, want, terms):
         assert float((a.double() - e).norm()) <= 4 * 2.0 ** -24 * (n + 1) ** 0.5 * float(e.norm()) + 1e-12
+
+
+@pytest.mark.parametrize("N,C,H,W,OC,k,s,p,d", [(2, 7, 9, 11, 16, 3, 1, 1, 1), (1, 16, 13, 8, 49, 3, 2, 1, 1),
+                                                (2, 24, 10, 10, 72, (3, 1), 1, 1, 2), (1, 64, 33, 5, 48, 1, 1, 0, 1)])
+def test_bf16_lowered_convolution(N, C, H, W, OC, k, s, p, d):
+    """The patch matrix (exact: it only moves values) and both ways of the input gradient, on either side of the filter
+    count where they change; results rounded to bf16."""
+    kh, kw = (k, k) if isinstance(k, int) else k
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    r = lambda *shape: torch.randn(*shape, generator=gen, device="cuda").bfloat16()
+    x, w = r(N, C, H, W), r(OC, C, kh, kw)
+    for dtype in (torch.bfloat16, torch.float32):
+        K = C * kh * kw
+        for ldc in (K, (K + 7) // 8 * 8, K + 3):
+            cols = cv.im2col(x.to(dtype), (kh, kw), s, p, d, ldc=ldc)
+            want = tF.unfold(x.float(), (kh, kw), d, p, s).transpose(1, 2).reshape(-1, K)
+            assert torch.equal(cols[:, :K].float(), want) and not cols[:, K:].any()
+    x.requires_grad_(), w.requires_grad_()
+    y = cv.conv2d(x, w, None, s, p, d)
+    dy = r(*y.shape)
+    got = [y, *torch.autograd.grad(y, [x, w], dy)]
+    x64, w64 = (v.detach().double().requires_grad_() for v in (x, w))
+    y64 = tF.conv2d(x64, w64, None, s, p, d)
+    for a, e in zip(got, [y64, *torch.autograd.grad(y64, [x64, w64], dy.double())]):
+        # 2^-9 for the result's rounding; the product route rounds k * k terms of each gradient as well
+        assert float((a.double() - e).norm()) <= 2.0 ** -7.5 * float(e.norm())
