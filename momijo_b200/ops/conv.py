@@ -101,9 +101,10 @@ def _channel_sum(dy, N, C, spatial):
 
 
 def _use_gemm(x, w, groups):
-    """bf16 with a contraction of at least 64 and a few thousand output positions: lower to the tensor cores."""
+    """Lower to the tensor cores: bf16 with a contraction of at least 64 and filters in eights, from sixteen on (the
+    product's rows are the filters, and it stores 16 bytes at a time); other counts run the direct kernels."""
     K = w.shape[1] * w.shape[2] * w.shape[3]
-    return x.dtype == bf16 and groups == 1 and K >= 64 and w.shape[0] >= 16
+    return x.dtype == bf16 and groups == 1 and K >= 64 and w.shape[0] >= 16 and w.shape[0] % 8 == 0
 
 
 class _Conv2d(torch.autograd.Function):

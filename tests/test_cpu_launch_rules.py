@@ -1,0 +1,13 @@
+"""Rules that pick a kernel, and launchers that refuse: host code, checked without a GPU."""
+import pytest
+import torch
+
+from momijo_b200.ops import conv
+
+
+@pytest.mark.parametrize("filters", [15, 16, 17, 20, 24, 48, 49, 56])
+def test_convolution_is_lowered_only_where_the_product_takes_its_filters(filters):
+    x = torch.zeros(1, 16, 8, 8, dtype=torch.bfloat16)
+    w = torch.zeros(filters, 16, 3, 3, dtype=torch.bfloat16)
+    # the product stores rows of filters 16 bytes at a time
+    assert conv._use_gemm(x, w, 1) == (filters >= 16 and filters % 8 == 0)
