@@ -825,6 +825,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   __shared__ __align__(8) uint64_t full_bar[kGemmMaxStages];
   __shared__ __align__(8) uint64_t empty_bar[kGemmMaxStages];
   __shared__ __align__(8) uint64_t done_bar[kGemmMaxStages];   // kMode 5: the stage's products have read it
+  __shared__ __align__(8) uint64_t sums_bar[2];                // kMode 5: the warps' sums are written / have been read
   __shared__ __align__(8) uint64_t tfull_bar[2];
   __shared__ __align__(8) uint64_t tempty_bar[2];
   __shared__ uint32_t tmem_slot;
@@ -844,6 +845,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], kMode == 5 ? kEpiWarps : 1);
       if (kMode == 5) mbar_init(&done_bar[s], 1);
+    }
+    if (kMode == 5) {
+      mbar_init(&sums_bar[0], kEpiWarps);
+      mbar_init(&sums_bar[1], kEpiWarps / 2);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
@@ -973,7 +978,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       int acc = 0;
       uint32_t acc_ph = 0;
       int cs = 0;          // kMode 5: the stage whose columns come next
-      uint32_t cph = 0;
+      uint32_t cph = 0, sph = 0;
       for (int t = pair; t < num_tiles; t += num_pairs) {
         const KRange kr = krange_of(t, per_group, num_k, p);
         const TileCoord tc = tile_of(kr.tt, num_m, num_n, p);
@@ -1004,22 +1009,32 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
             if (lane == 0) mbar_arrive(&empty_bar[cs]);
             if (++cs == stages) { cs = 0; cph ^= 1; }
           }
-          if (tc.n_tile == 0) {   // (after a timeout too: every epilogue warp meets at the barriers)
+          if (!ok) break;
+          if (tc.n_tile == 0) {
+            // The warps meet on mbarriers: a warp that gives up leaves this loop alone, on any tile, and the others then
+            // run out of time as well, where a named barrier would wait for it for good.
             total = f2_add(total, part);
             float* mine = reinterpret_cast<float*>(epi_stage[warp - 2]);
             f2_unpack(total, mine[2 * lane], mine[2 * lane + 1]);
-            asm volatile("bar.sync 1, 256;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sums_bar[0]);
             const int c = (int)threadIdx.x - 64;
-            if (c < 128 && m0 + c < p.M) {
-              float v = 0.f;
+            if (c < 128) {   // four of the eight warps
+              if (!mbar_wait_warp(&sums_bar[0], sph, &abort_flag, p.status, kTimeoutFlag, t)) break;
+              if (m0 + c < p.M) {
+                float v = 0.f;
 #pragma unroll
-              for (int q = 0; q < kEpiWarps / 2; ++q)
-                v += reinterpret_cast<const float*>(epi_stage[(c >> 6) + 2 * q])[c & 63];
-              p.bias_part[(long long)kr.g * p.M + m0 + c] = v;
+                for (int q = 0; q < kEpiWarps / 2; ++q)
+                  v += reinterpret_cast<const float*>(epi_stage[(c >> 6) + 2 * q])[c & 63];
+                p.bias_part[(long long)kr.g * p.M + m0 + c] = v;
+              }
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&sums_bar[1]);
             }
-            asm volatile("bar.sync 1, 256;" ::: "memory");
+            // the staging areas are free again
+            if (!mbar_wait_warp(&sums_bar[1], sph, &abort_flag, p.status, kTimeoutFlag, t)) break;
+            sph ^= 1;
           }
-          if (!ok) break;
         }
         if (kr.nk == 0) {
           const int zrow = m0 + quad * 32 + lane;
