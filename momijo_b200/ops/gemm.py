@@ -76,7 +76,7 @@ def pick_bn(M: int, N: int) -> int:
     return best
 
 
-_SPLITK = {"ranges": {}, "scratch": None, "enabled": True, "force": None}
+_SPLITK = {"ranges": {}, "enabled": True, "force": None}
 
 
 # Measured cost of one 64-deep K block of a tile, in SM cycles (B200, operands streamed from L2/HBM):
@@ -167,14 +167,6 @@ def _split_ranges(K: int, S: int, device):
     return r
 
 
-def _slabs(need, device):
-    sc = _SPLITK["scratch"]
-    if sc is None or sc.numel() < need or sc.device != device:
-        sc = torch.empty(need, dtype=torch.float32, device=device)
-        _SPLITK["scratch"] = sc
-    return sc
-
-
 def wgrad_bias(dy, x, out, accumulate, db, db_accumulate) -> bool:
     """``out (+)= dy^T x`` and ``db (+)= column sums of dy`` in one product where the weight gradient is split over CTA
     pairs; False (and nothing done) where it is not."""
@@ -187,7 +179,8 @@ def wgrad_bias(dy, x, out, accumulate, db, db_accumulate) -> bool:
     if S <= 1 or tall != "pair":
         return False
     lddy, ldx = _check_2d(dy, "a"), _check_2d(x, "b")
-    sc = _slabs(S * M * N, dy.device)
+    # slabs of this call's own: calls on other streams or threads run between the product and its fold
+    sc = dy.new_empty(S * M * N, dtype=torch.float32)
     part = dy.new_empty(S * M, dtype=torch.float32)
     _C.call("mmj_wgrad_bias", dy.data_ptr(), lddy, x.data_ptr(), ldx, sc.data_ptr(), part.data_ptr(), K, M, N, S,
             _C.ptr(_split_ranges(K, S, dy.device)), _C.status_tensor(dy.device).data_ptr(), _C.current_stream())
@@ -199,7 +192,7 @@ def wgrad_bias(dy, x, out, accumulate, db, db_accumulate) -> bool:
 
 def _gemm_split_k(a, b, out, accumulate, M, N, K, S, bn, tall=False):
     """a: [K, M], b: [K, N] (both MN-major). Partial products as fp32 slabs, then one reduction pass."""
-    sc = _slabs(S * M * N, a.device)
+    sc = a.new_empty(S * M * N, dtype=torch.float32)   # of this call's own, as in wgrad_bias
     _C.call("mmj_gemm_bf16_grouped_k", _C.ptr(a), a.stride(0), _C.ptr(b), b.stride(0), _C.ptr(sc), N, K, M, N, S,
             _C.ptr(_split_ranges(K, S, a.device)), 1, 0,
             bn | (PAIR if tall == "pair" else TALL if tall else 0),
