@@ -1579,13 +1579,15 @@ static int epilogue_vec_ok(const GemmParams& p) {
   return ok ? 1 : 0;
 }
 
-// Split kernel launcher: plain products with K-major A. `splits`: 1, 2, 4 or 8 ranges of K.
+// Split kernel launcher: plain products with K-major A. `splits`: 1, 2, 4 or 8 ranges of K, none of them empty (a CTA
+// without a K block would commit no accumulator, and its peers would add a partial tile that was never written).
 int launch_gemm_split(GemmParams& p, const void* A, long long lda, long long a_rows, const void* B, long long ldb,
                       long long b_rows, int splits, cudaStream_t stream) {
   if (p.M <= 0 || p.N <= 0) return 0;
   if ((lda % 8) != 0 || (ldb % 8) != 0) return -2;
   if (((uintptr_t)A & 15) || ((uintptr_t)B & 15)) return -3;
   if (p.a_mn || (p.epi & kEpiScatterPeers) || p.K <= 0) return -7;
+  if (splits < 1 || splits > 8 || (splits & (splits - 1)) || splits > (p.K + kGemmBK - 1) / kGemmBK) return -4;
   p.vec_ok = epilogue_vec_ok(p);
   CUtensorMap tmA, tmB;
   int rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)p.K, (uint64_t)a_rows, (uint64_t)lda, 64, 128);
@@ -1600,9 +1602,7 @@ int launch_gemm_split(GemmParams& p, const void* A, long long lda, long long a_r
   SplitKernel kernel = splits == 1   ? &gemm_bf16_split_kernel<1>
                        : splits == 2 ? &gemm_bf16_split_kernel<2>
                        : splits == 4 ? &gemm_bf16_split_kernel<4>
-                       : splits == 8 ? &gemm_bf16_split_kernel<8>
-                                     : nullptr;
-  if (kernel == nullptr) return -4;
+                                     : &gemm_bf16_split_kernel<8>;
   static bool attr_set = false;
   if (!attr_set) {
     for (SplitKernel k : {&gemm_bf16_split_kernel<1>, &gemm_bf16_split_kernel<2>, &gemm_bf16_split_kernel<4>,

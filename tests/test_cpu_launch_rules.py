@@ -61,3 +61,20 @@ def test_split_weight_gradients_of_two_streams_share_no_slabs(monkeypatch, fused
     slabs = [c[1][4] for c in calls if c[0] == product]
     assert slabs[0] != slabs[1]
     assert [c[1][0] for c in calls if c[0] == fold] == [slabs[1], slabs[0]]
+
+
+@pytest.mark.parametrize("k,splits", [(64, 2), (64, 8), (128, 4), (200, 8), (448, 8), (512, 3), (512, 0), (4096, 16)])
+def test_split_launcher_refuses_empty_ranges(k, splits):
+    """Refused before anything is launched (or asked of a driver): more ranges than 64-deep blocks, or a count that no
+    kernel exists for."""
+    operand = 4096   # a 16-byte aligned address that nothing reads
+    rc = _C.lib().mmj_gemm_bf16(operand, k, 0, operand, k, 0, operand, 64, 128, 64, k, 0, None, None, 0, None, 0, None,
+                                gemm_mod.SPLIT | splits << 16, None, None)
+    assert rc == -4
+
+
+def test_split_rule_leaves_no_range_empty():
+    for m in (1, 100, 128, 129, 255, 256, 700):
+        for n in (8, 64, 72, 520, 2304):
+            for k in (8, 64, 448, 512, 520, 576, 1024, 4096):
+                assert gemm_mod.pick_split(m, n, k) <= -(-k // 64)
