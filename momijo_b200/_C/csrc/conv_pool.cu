@@ -247,7 +247,8 @@ __global__ void __launch_bounds__(256) conv2d_dw_kernel(const T* __restrict__ x,
 // (offset, row and column shift, weight offset) computed once per block by 16 threads, two chunks ahead.
 // Measured at that shape, before -> now: forward 4121 -> 217 us (34 TFLOP/s), input gradient 10160 -> 216 us; three
 // blocks per SM (168 registers, no spills) against four: 217 / 224 us.
-// Taps outside the image are multiplied as zeros, as zero padding is in torch.
+// Taps outside the image are multiplied as zeros. An infinite weight would make a NaN of those, where the tap does not
+// exist: results that come out as NaN are computed again by skip_sum, without such taps.
 struct GatherGeom {
   int SH, SW;                      // image that is gathered from
   int cls_h, cls_w;                // pixel classes (strides of an input gradient; 1 x 1 in a forward pass)
@@ -289,10 +290,54 @@ __device__ __forceinline__ AxisTaps axis_taps(int transposed, int cls, int strid
 
 constexpr int kGatherBN = 128, kGatherBK = 16, kGatherThreads = 128;
 
+// One result of the tiled product, in its order, over the taps inside the image only; false where every tap is inside.
+// `sp` points at the position's source pixel (h0, w0), `wp` at the output channel's weights.
+template <typename T>
+__device__ bool skip_sum(const T* sp, const T* wp, const GatherGeom& g, const AxisTaps& vh, const AxisTaps& vw, int h0,
+                         int w0, float& sum) {
+  bool outside = false;
+  float s = 0.f;
+  for (int ch = 0; ch < g.channels; ++ch)
+    for (int ih = 0; ih < vh.count; ++ih)
+      for (int iw = 0; iw < vw.count; ++iw) {
+        const int eh = vh.e0 + ih * vh.es, ew = vw.e0 + iw * vw.es;
+        if ((unsigned)(h0 + eh) >= (unsigned)g.SH || (unsigned)(w0 + ew) >= (unsigned)g.SW) {
+          outside = true;
+          continue;
+        }
+        if (ch > 0 && !outside) return false;
+        s = fmaf(to_f<T>(wp[ch * (int)g.w_ch + (vh.first + ih * vh.step) * g.kW + (vw.first + iw * vw.step)]),
+                 to_f<T>(sp[ch * g.SH * g.SW + eh * g.SW + ew]), s);
+      }
+  sum = s;
+  return outside;
+}
+// The NaNs among one thread's results, in a function of its own so that the product's registers don't know of it.
+template <typename T, int TM, int TN>
+__device__ __noinline__ void skip_nan_results(const T* src, const T* wt, const T* bias, T* dst, const long long* out_off,
+                                              const GatherGeom& g, long long p0, int grp, int mt, int tx, int ca, int cb) {
+  const int PH = (g.PHf - ca + g.cls_h - 1) / g.cls_h, PW = (g.PWf - cb + g.cls_w - 1) / g.cls_w;
+  const AxisTaps vh = axis_taps(g.transposed, ca, g.cls_h, g.kH, g.dh, g.ph);
+  const AxisTaps vw = axis_taps(g.transposed, cb, g.cls_w, g.kW, g.dw, g.pw);
+  for (int i = 0; i < TM * TN; ++i) {
+    const int m = mt + i / TN, jj = i % TN;
+    const int p = (jj >> 2) * (kGatherBN * 4 / TN) + tx * 4 + (jj & 3);
+    if (m >= g.M || out_off[p] < 0) continue;
+    T* o = dst + (long long)m * g.dst_m + out_off[p];
+    if (to_f<T>(*o) == to_f<T>(*o)) continue;
+    const long long pos = p0 + p, q = pos / PW;
+    const int h = (int)(q % PH) * g.pos_s_h + g.pos_o_h, w = (int)(pos % PW) * g.pos_s_w + g.pos_o_w;
+    float v;
+    if (skip_sum<T>(src + q / PH * g.src_n + grp * g.src_g + (long long)h * g.SW + w, wt + grp * g.w_g + m * g.w_m, g, vh,
+                    vw, h, w, v))
+      *o = from_f<T>(v + ((bias != nullptr) ? to_f<T>(bias[grp * g.M + m]) : 0.f));
+  }
+}
+
 template <typename T, int BM, int TM, int TN>
 __global__ void __launch_bounds__(kGatherThreads, 3)
     conv_gather_kernel(const T* __restrict__ src, const T* __restrict__ wt, const T* __restrict__ bias,
-                       T* __restrict__ dst, GatherGeom g) {
+                       T* __restrict__ dst, const __grid_constant__ GatherGeom g) {
   constexpr int BN = kGatherBN, BK = kGatherBK;
   constexpr int TX = BN / TN, TY = BM / TM;
   static_assert(TX * TY == kGatherThreads, "tile and thread count disagree");
@@ -309,6 +354,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3)
   const long long P = (long long)g.N * PH * PW;
   const long long p0 = (long long)blockIdx.x * BN;
   if (p0 >= P) return;                           // classes differ by a row or a column
+  bool nan = false;
   const int m_tiles = (g.M + BM - 1) / BM;
   const int grp = (int)blockIdx.y / m_tiles, m0 = ((int)blockIdx.y % m_tiles) * BM;
   const AxisTaps vh = axis_taps(g.transposed, ca, g.cls_h, g.kH, g.dh, g.ph);
@@ -436,12 +482,15 @@ __global__ void __launch_bounds__(kGatherThreads, 3)
       f2_unpack(acc[i][j], lo, hi);
       if (out_off[p] >= 0) o[out_off[p]] = from_f<T>(lo + bv);
       if (out_off[p + 1] >= 0) o[out_off[p + 1]] = from_f<T>(hi + bv);
+      nan |= (lo != lo) | (hi != hi);
     }
   }
+  if (nan)
+    skip_nan_results<T, TM, TN>(src, wt, bias, dst, out_off, g, p0, grp, m0 + ty * TM, tx, ca, cb);
 }
 
 // Weight gradient: dw[oc, k] = sum_p dy[oc, p] * x(k, p), both operands contiguous along p. A block owns a
-// BM x 64 tile of dw and one slice of the positions; slices write fp32 slabs that wgrad_fold_kernel adds in slice
+// BM x 64 tile of dw and one slice of the positions; slices write fp32 slabs that slab_fold_kernel adds in slice
 // order, so that results stay bitwise reproducible. A thread adds at most 64 products in a row before it folds
 // them into a second sum, so that chains stay as short as in the direct kernel's 256-thread block sum (error against
 // 64 bits at N32 C64 56x56 OC64 k3: 3.6e-7 before, 1.9e-7 now). The direct kernel re-read both images for each of its
@@ -584,16 +633,50 @@ __global__ void __launch_bounds__(kWgThreads, 4)
   }
 }
 
-// dst[i] = sum over S slabs: 8 lanes of slabs per element group, folded in a fixed order
+// The tiles multiply pixels outside the image as zeros, which an infinite dy turns into NaN where the tap does not exist:
+// a NaN sum of one slice [pb, pe) again without such pixels, in chains of 64 as well. i: (filter, channel, tap).
 template <typename T>
-__global__ void __launch_bounds__(256) wgrad_fold_kernel(const float* __restrict__ slabs, T* __restrict__ dst,
-                                                         long long n, int S) {
+__device__ __noinline__ float wgrad_skip_sum(const T* x, const T* dy, const ConvGeom& g, long long i, long long pb,
+                                             long long pe, float nan) {
+  const int cg = g.C / g.groups, taps = g.kH * g.kW, K = cg * taps, spatial = g.OH * g.OW;
+  const int oc = (int)(i / K), k = (int)(i - (long long)oc * K), ch = k / taps, t = k - ch * taps;
+  const int eh = t / g.kW * g.dh - g.ph, ew = t % g.kW * g.dw - g.pw;
+  if (eh >= 0 && (g.OH - 1) * g.sh + eh < g.H && ew >= 0 && (g.OW - 1) * g.sw + ew < g.W) return nan;   // never outside
+  const T* xc = x + (long long)(oc / (g.OC / g.groups) * cg + ch) * g.H * g.W;
+  float total = 0.f, part = 0.f;
+  for (long long p = pb; p < pe; ++p) {
+    const int n = (int)(p / spatial), s = (int)(p - (long long)n * spatial);
+    const int h = s / g.OW * g.sh + eh, w = s % g.OW * g.sw + ew;
+    if ((unsigned)h < (unsigned)g.H && (unsigned)w < (unsigned)g.W)
+      part = fmaf(to_f<T>(dy[((long long)n * g.OC + oc) * spatial + s]),
+                  to_f<T>(xc[(long long)n * g.C * g.H * g.W + (long long)h * g.W + w]), part);
+    if (((p - pb) & 63) == 63) {
+      total += part;
+      part = 0.f;
+    }
+  }
+  return total + part;
+}
+
+// dst[i] = sum over S slabs: 8 lanes of slabs per element group, folded in a fixed order. kConv: slabs of a weight
+// gradient over slices of `slice` positions.
+template <typename T, bool kConv>
+__global__ void __launch_bounds__(256) slab_fold_kernel(const float* __restrict__ slabs, T* __restrict__ dst, long long n,
+                                                        int S, const T* __restrict__ x, const T* __restrict__ dy,
+                                                        const __grid_constant__ ConvGeom g, long long slice) {
   __shared__ float part[8][32];
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
   const long long i = (long long)blockIdx.x * 32 + lane;
   float a = 0.f;
   if (i < n)
-    for (int s = row; s < S; s += 8) a += slabs[(long long)s * n + i];
+    for (int s = row; s < S; s += 8) {
+      float v = slabs[(long long)s * n + i];
+      if (kConv && v != v) {
+        const long long pb = s * slice, P = (long long)g.N * g.OH * g.OW;
+        v = wgrad_skip_sum<T>(x, dy, g, i, pb, pb + slice < P ? pb + slice : P, v);
+      }
+      a += v;
+    }
   part[row][lane] = a;
   __syncthreads();
   if (row == 0 && i < n) {
@@ -604,7 +687,7 @@ __global__ void __launch_bounds__(256) wgrad_fold_kernel(const float* __restrict
 }
 
 // db[oc] = sum_{n, oh, ow} dy[n, oc, oh, ow]: `splits` blocks per channel over whole images (one block per channel
-// left 84 of 148 SMs idle at 64 channels: 223 us for 25.7 MB), folded in order by wgrad_fold_kernel.
+// left 84 of 148 SMs idle at 64 channels: 223 us for 25.7 MB), folded in order by slab_fold_kernel.
 template <typename T>
 __global__ void __launch_bounds__(256) channel_sum_kernel(const T* __restrict__ dy, float* __restrict__ part, int N,
                                                           int OC, long long spatial, int splits) {
@@ -910,7 +993,8 @@ static int launch_wgrad(const void* x, const void* dy, void* dw, float* scratch,
   if (bm == 64) conv_wgrad_kernel<T, 64><<<grid, kWgThreads, 0, st>>>((const T*)x, (const T*)dy, scratch, g, len);
   else if (bm == 32) conv_wgrad_kernel<T, 32><<<grid, kWgThreads, 0, st>>>((const T*)x, (const T*)dy, scratch, g, len);
   else conv_wgrad_kernel<T, 16><<<grid, kWgThreads, 0, st>>>((const T*)x, (const T*)dy, scratch, g, len);
-  wgrad_fold_kernel<T><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(scratch, (T*)dw, n, S);
+  slab_fold_kernel<T, true><<<(unsigned)((n + 31) / 32), 256, 0, st>>>(scratch, (T*)dw, n, S, (const T*)x, (const T*)dy, g,
+                                                                     len);
   return (int)cudaGetLastError();
 }
 MMJ_API int mmj_conv2d_dw(const void* x, const void* dy, void* dw, float* scratch, const int* geom, int dtype,
@@ -944,8 +1028,11 @@ MMJ_API int mmj_channel_sum(const void* dy, void* db, float* scratch, int N, int
   DISPATCH(dtype, (channel_sum_kernel<float><<<grid, 256, 0, STREAM>>>((const float*)dy, scratch, N, OC, spatial, S)),
            (channel_sum_kernel<__nv_bfloat16><<<grid, 256, 0, STREAM>>>((const __nv_bfloat16*)dy, scratch, N, OC,
                                                                         spatial, S)));
-  DISPATCH(dtype, (wgrad_fold_kernel<float><<<(OC + 31) / 32, 256, 0, STREAM>>>(scratch, (float*)db, OC, S)),
-           (wgrad_fold_kernel<__nv_bfloat16><<<(OC + 31) / 32, 256, 0, STREAM>>>(scratch, (__nv_bfloat16*)db, OC, S)));
+  const ConvGeom none = {};
+  DISPATCH(dtype, (slab_fold_kernel<float, false><<<(OC + 31) / 32, 256, 0, STREAM>>>(scratch, (float*)db, OC, S, nullptr,
+                                                                                      nullptr, none, 0)),
+           (slab_fold_kernel<__nv_bfloat16, false><<<(OC + 31) / 32, 256, 0, STREAM>>>(scratch, (__nv_bfloat16*)db, OC, S,
+                                                                                       nullptr, nullptr, none, 0)));
   return (int)cudaGetLastError();
 }
 

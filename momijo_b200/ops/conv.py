@@ -101,8 +101,8 @@ def _channel_sum(dy, N, C, spatial):
 
 
 def _use_gemm(x, w, groups):
-    """Lower to the tensor cores: bf16 with a contraction of at least 64 and filters in eights, from sixteen on (the
-    product's rows are the filters, and it stores 16 bytes at a time); other counts run the direct kernels."""
+    """Lower to the tensor cores: bf16 with a contraction of at least 64 and filters in eights, from sixteen on (they
+    are the product's columns, which it stores 16 bytes at a time); other counts run the direct kernels."""
     K = w.shape[1] * w.shape[2] * w.shape[3]
     return x.dtype == bf16 and groups == 1 and K >= 64 and w.shape[0] >= 16 and w.shape[0] % 8 == 0
 

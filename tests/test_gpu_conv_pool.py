@@ -158,3 +158,47 @@ def test_bf16_lowered_convolution(N, C, H, W, OC, k, s, p, d):
     for a, e in zip(got, [y64, *torch.autograd.grad(y64, [x64, w64], dy.double())]):
         # 2^-9 for the result's rounding; the product route rounds k * k terms of each gradient as well
         assert float((a.double() - e).norm()) <= 2.0 ** -7.5 * float(e.norm())
+
+
+def _taps_by_slices(x, w, dy, s, p, d):
+    """y, dx and dw of a convolution as sums over the taps that lie inside the image, in 64 bits: nothing is multiplied
+    by a padding zero."""
+    x, w, dy = x.double().cpu(), w.double().cpu(), dy.double().cpu()
+    y, dx, dw = torch.zeros_like(dy), torch.zeros_like(x), torch.zeros_like(w)
+    (OH, OW), (H, W) = dy.shape[2:], x.shape[2:]
+    for kh in range(w.shape[2]):
+        for kw in range(w.shape[3]):
+            rows = [(o, o * s - p + kh * d) for o in range(OH) if 0 <= o * s - p + kh * d < H]
+            cols = [(o, o * s - p + kw * d) for o in range(OW) if 0 <= o * s - p + kw * d < W]
+            if not rows or not cols:
+                continue
+            o = (..., slice(rows[0][0], rows[-1][0] + 1), slice(cols[0][0], cols[-1][0] + 1))
+            i = (..., slice(rows[0][1], rows[-1][1] + 1, s), slice(cols[0][1], cols[-1][1] + 1, s))
+            y[o] += (x[i][:, None] * w[None, :, :, kh, kw, None, None]).sum(2)
+            dx[i] += (dy[o][:, :, None] * w[None, :, :, kh, kw, None, None]).sum(1)
+            dw[:, :, kh, kw] += (dy[o][:, :, None] * x[i][:, None]).sum((0, 3, 4))
+    return y, dx, dw
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,s,p,d", [(14, 1, 1, 1), (37, 2, 1, 1), (37, 1, 2, 2), (60, 3, 2, 1), (40, 1, 1, 1)])
+def test_infinite_values_meet_only_taps_inside_the_image(dtype, H, s, p, d):
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    N, C, OC, k = 3, 4, 5, 3
+    OH = (H + 2 * p - d * (k - 1) - 1) // s + 1
+    r = lambda *shape: torch.randn(*shape, generator=gen, device="cuda").to(dtype)
+    x, w, dy = r(N, C, H, H), r(OC, C, k, k), r(N, OC, OH, OH)
+    inf_w = w.clone()
+    inf_w[2, 1, 0, 2] = float("inf")           # a corner tap: outside the image for a row and a column of pixels
+    inf_dy = dy.clone()
+    inf_dy[1, 3, 0, OH - 1] = float("-inf")    # a corner pixel: some of its taps are outside
+    for wt, grad in ((inf_w, dy), (w, inf_dy)):
+        xg, wg = x.clone().requires_grad_(), wt.clone().requires_grad_()
+        y = cv.conv2d(xg, wg, None, s, p, d)
+        got = [y, *torch.autograd.grad(y, [xg, wg], grad)]
+        for a, e in zip(got, _taps_by_slices(x, wt, grad, s, p, d)):
+            a, fin = a.detach().double().cpu(), torch.isfinite(e)
+            assert torch.equal(torch.isnan(a), torch.isnan(e)) and torch.equal(a[~fin], e[~fin])
+            # sums of up to n products: 4 * 2^-24 * sqrt(n) of the norm, and 2^-8 for a bf16 result
+            tol = 4 * 2.0 ** -24 * (N * OH * OH) ** 0.5 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+            assert float((a - e)[fin].norm()) <= tol * float(e[fin].norm())
