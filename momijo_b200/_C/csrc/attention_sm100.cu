@@ -38,6 +38,8 @@ struct AttnParams {
   float* lse;  // [B, Hq, T]
   // backward
   const float* delta;  // [B, Hq, T]
+  float scale_log2;    // scale * log2(e); a factor too small to reach a sum where scale is 0
+  uint32_t dead_score; // bits of the infinity that scale_log2 turns into -inf
   float* dQ;           // fp32 accumulator [B*T, ld_dq]
   long long ld_dq;
   __nv_bfloat16* dK;
@@ -897,7 +899,9 @@ struct BwdCfg {
   static constexpr int kThreads = (8 + 8 * kGroups) * 32;
 };
 
-template <int D>
+// kPositive: the scale is positive, as nearly always; the other form's two parameters cost registers that head_dim 64 does
+// not have to spare.
+template <int D, bool kPositive>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -1181,7 +1185,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int row = quad * 32 + lane;
     const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
     const float l2e = 1.4426950408889634f;
-    const f32x2 c2 = f2_pack(p.scale * l2e, p.scale * l2e);
+    const f32x2 c2 = kPositive ? f2_pack(p.scale * l2e, p.scale * l2e) : f2_pack(p.scale_log2, p.scale_log2);
     float* my_lse = ctl.neg_lse[warp - 4];
     float* my_delta = ctl.neg_delta[warp - 4];
     // position in the CTA's sequence of blocks
@@ -1256,7 +1260,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_ld_cols(t_lane + col, rs);
         tmem_ld_cols(t_lane + col + 64, rp);
         tmem_ld_wait();
-        // Queries below the key row (causal) and key rows past the end have P = 0: their scores become -inf. (A
+        // Queries below the key row (causal) and key rows past the end have P = 0: their scaled scores become -inf. (A
         // second, masked copy of the block below ran twice an item, each time from a cold instruction cache, and took
         // 2000 cycles longer than the plain one.)
         const int lim = p.causal ? kv_idx - (cur.qi * 64 + chalf * 32 + sub * kCols) : 0;   // columns below it are dead
@@ -1264,7 +1268,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (__any_sync(0xffffffffu, (lim > 0) | past)) {
           const uint32_t live = (past || lim >= kCols) ? 0u : lim <= 0 ? 0xffffffffu : 0xffffffffu << lim;
 #pragma unroll
-          for (int i = 0; i < kCols; ++i) rs[i] = (live & (1u << i)) ? rs[i] : 0xff800000u;
+          for (int i = 0; i < kCols; ++i) rs[i] = (live & (1u << i)) ? rs[i] : kPositive ? 0xff800000u : p.dead_score;
         }
         uint32_t pw[kCols];   // P^T as bf16 pairs, then dS^T
 #pragma unroll
@@ -1559,6 +1563,8 @@ MMJ_API int mmj_attn_bwd(const void* q, long long ldq, int q_col0, const void* k
   p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;
   p.o_col0 = do_col0;  // the dO map is addressed with o_col0 inside the kernel
   p.scale = scale; p.causal = causal;
+  p.scale_log2 = scale == 0.f ? 1e-30f : scale * 1.4426950408889634f;
+  p.dead_score = scale < 0.f ? 0x7f800000u : 0xff800000u;
   p.lse = const_cast<float*>(lse);
   p.delta = delta;
   p.dQ = dQ_accum; p.ld_dq = ld_dq; p.dq_col0 = dq_col0;
@@ -1576,9 +1582,11 @@ MMJ_API int mmj_attn_bwd(const void* q, long long ldq, int q_col0, const void* k
   // head_dim 128: 224 KB of tiles, the control block and the alignment padding take what is left of the 227 KB a CTA
   // may have (the kernel checks that they fit); head_dim 64 needs 208 KB of tiles
   const int smem = 232448;
-  static bool attr64 = false, attr128 = false;
-  bool& attr = (D == 64) ? attr64 : attr128;
-  auto* kernel = (D == 64) ? &attn_bwd_kernel<64> : &attn_bwd_kernel<128>;
+  static bool attr_set[4] = {};
+  const bool positive = scale > 0.f;
+  auto* kernel = (D == 64) ? (positive ? &attn_bwd_kernel<64, true> : &attn_bwd_kernel<64, false>)
+                           : (positive ? &attn_bwd_kernel<128, true> : &attn_bwd_kernel<128, false>);
+  bool& attr = attr_set[(D == 64 ? 0 : 2) + (positive ? 1 : 0)];
   if (!attr) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     attr = true;

@@ -381,6 +381,27 @@ def test_attention_backward_block_edges(B, T, Hq, Hkv, D, causal):
     assert torch.isfinite(got).all()
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.1, 0.3])
+@pytest.mark.parametrize("T,D", [(64, 64), (192, 64), (192, 128), (256, 128)])
+def test_attention_backward_of_any_scale(T, D, scale):
+    """Key rows past the end of the last key block take no part, whatever the sign of the scale (0: equal weights)."""
+    torch.manual_seed(12)
+    qkv, dy = _rand(2 * T, 4 * D, grad=True), _rand(2 * T, 2 * D)
+    y = ops.attention_packed(qkv, 2, T, 2, 1, D, causal=False, scale=scale)
+    (got,) = torch.autograd.grad(y, qkv, dy)
+    x = qkv.detach().double().cpu().requires_grad_()
+    v = x.view(2, T, 4, D).transpose(1, 2)
+    p = torch.softmax(v[:, :2] @ v[:, 2:3].transpose(-1, -2) * scale, -1)
+    ref = (p @ v[:, 3:]).transpose(1, 2).reshape(2 * T, 2 * D)
+    (want,) = torch.autograd.grad(ref, x, dy.double().cpu())
+    _close(y, ref.detach().cuda())
+    for lo, hi in ((0, 2), (2, 3), (3, 4)):
+        a, e = got[:, lo * D:hi * D], want[:, lo * D:hi * D].cuda()
+        assert not a.any() if scale == 0.0 and lo < 3 else True     # dQ and dK carry the scale as a factor
+        if scale != 0.0 or lo == 3:
+            _close(a, e)
+
+
 @pytest.mark.parametrize("B,T,Hq,Hkv,D", [(2, 37, 2, 1, 64), (1, 130, 4, 4, 128), (3, 5, 6, 2, 128)])
 def test_attention_rotary_paths(B, T, Hq, Hkv, D):
     """Rotation fused into the copy of the packed rows and into the gradient's cast, a misaligned input view among
