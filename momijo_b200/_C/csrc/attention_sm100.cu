@@ -99,7 +99,7 @@ __device__ __forceinline__ void bulk_wait_group0() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// Optional timeline of the forward kernels: when a trace buffer is installed, one softmax thread and the
+// Optional kernel timeline: when a trace buffer is installed, one softmax (or compute) thread and the
 // MMA thread of every CTA store clock64() stamps at their stage boundaries (64 slots per CTA).
 constexpr int kTraceSlots = 64;
 __device__ __forceinline__ void trace_stamp(long long* trace, int cta, int slot) {
@@ -899,9 +899,12 @@ struct BwdCfg {
   static constexpr int kThreads = (8 + 8 * kGroups) * 32;
 };
 
-// kPositive: the scale is positive, as nearly always; the other form's two parameters cost registers that head_dim 64 does
-// not have to spare.
-template <int D, bool kPositive>
+// kPlain: the scale is positive and no timeline is recorded, as nearly always; what the other form needs costs registers
+// that head_dim 64 does not have to spare. Its timeline: slot 0 start, 1 SM, 2 set up, 3 K / V landed (score issuer),
+// 4 first dK / dV complete, 5 first compute warp done, 6 end, 7 blocks of the first item; block g of the CTA's sequence,
+// g < 9: 8 + 6 g + 0 scores seen, 1 read from TMEM, 2 P^T and dS^T stored (first warp of the block's
+// compute group), 3 dQ^T seen, 4 its reduce-add issued (drain warp), 5 P^T and dS^T seen by the gradient issuer.
+template <int D, bool kPlain>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -954,7 +957,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   };
   auto first_block = [&](int w) -> int { return p.causal ? 2 * (w / n_heads_b) : 0; };
 
+  // slots past the last recorded block fall off the end of the CTA's row
+  auto stamp = [&](int slot) {
+    if constexpr (!kPlain) trace_stamp(p.trace, cta, slot);
+  };
+  auto stamp_block = [&](uint32_t g, int what) {
+    if constexpr (!kPlain) trace_stamp(p.trace, cta, g < 9u ? 8 + 6 * (int)g + what : kTraceSlots);
+  };
   if (threadIdx.x == 0) {
+    stamp(0);
+    if (!kPlain && p.trace != nullptr) {
+      uint32_t smid;
+      asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+      p.trace[(long long)cta * kTraceSlots + 1] = smid;
+      p.trace[(long long)cta * kTraceSlots + 7] = (num_qb - first_block(item_at(0))) * group;
+    }
     mbar_init(&ctl.acc_full, 1);
     mbar_init(&ctl.acc_empty, kBufs == 3 ? 4 : 8 * kGroups);
     for (int s = 0; s < 2; ++s) {
@@ -990,6 +1007,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr uint32_t tmem_base = 0;   // an allocation of all 512 columns starts at column 0
   pdl_wait();  // the set-up above read no tensor of the step
   pdl_trigger();
+  if (threadIdx.x == 0) stamp(2);
 
   // dV / dK of item n: 32 key rows (one per lane), 32-column chunks [c0, c1) of head_dim. With one accumulator the
   // compute warps do this; with two the drain warps do, while the compute warps are already at the next item.
@@ -998,6 +1016,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   auto store_grads = [&](int quad, int c0, int c1, uint32_t n, int jb, int hkv, int b, uint8_t* st) -> bool {
     if (!mbar_wait_warp(&ctl.acc_full, n & 1, &abort_flag, p.status, kTimeoutTmemFull, 700)) return false;
     tc_fence_after();
+    if (n == 0 && quad == 0 && c0 == 0 && lane == 0) stamp(4);
     const int row0 = jb * 128 + quad * 32;
     const uint32_t colV = ((uint32_t)(quad * 32) << 16) + kColV;
     __nv_bfloat16* dk = p.dK + ((long long)b * p.T + row0) * p.ld_dk + p.dk_col0 + hkv * D;
@@ -1098,6 +1117,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t kb = n % kKV;
       const int n_iter = (num_qb - first_block(w)) * group;
       if (!mbar_wait_warp(&ctl.kv_full[kb], (n / kKV) & 1, &abort_flag, p.status, kTimeoutFull, 1001)) break;
+      if (n == 0 && lane == 0) stamp(3);
       ++n;
       const uint32_t ak = lo_k + kb * (2 * kTile >> 4);
       for (int it = 0; it < n_iter; ++it, ++g) {
@@ -1144,6 +1164,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (!mbar_wait_warp(&ctl.qdo_full[s], ph, &abort_flag, p.status, kTimeoutFull, (int)g) ||
             !mbar_wait_warp(&ctl.pds_full[bf], bph, &abort_flag, p.status, kTimeoutFlag, (int)g)) { ok = false; break; }
         tc_fence_after();
+        if (lane == 0) stamp_block(g, 5);
         const uint32_t bq = lo_qmn + s * (2 * kQTile >> 4);
         const uint32_t bds = lo_dsmn + bf * (kDsBytes >> 4);
         const uint32_t acc = it > 0 ? 1u : 0u;
@@ -1185,7 +1206,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int row = quad * 32 + lane;
     const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
     const float l2e = 1.4426950408889634f;
-    const f32x2 c2 = kPositive ? f2_pack(p.scale * l2e, p.scale * l2e) : f2_pack(p.scale_log2, p.scale_log2);
+    const f32x2 c2 = kPlain ? f2_pack(p.scale * l2e, p.scale * l2e) : f2_pack(p.scale_log2, p.scale_log2);
     float* my_lse = ctl.neg_lse[warp - 4];
     float* my_delta = ctl.neg_delta[warp - 4];
     // position in the CTA's sequence of blocks
@@ -1230,6 +1251,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     stat_load(ahead);
     uint32_t bf = grp, bph = 0;   // the block's buffer and its phase
     int stored = 0;   // items whose dV / dK this warp has stored (head_dim 128)
+    const bool tracer = !kPlain && ((warp - 4) & 7) == 0 && lane == 0;
+    uint32_t blk = grp;   // position in the CTA's sequence (timeline)
     bool ok = true;
     while (true) {
       if (kBufs == 2) {
@@ -1251,6 +1274,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       stat_load(ahead);
       if (!mbar_wait_warp(&ctl.s_full[bf], bph, &abort_flag, p.status, kTimeoutTmemFull, (int)bf)) break;
       tc_fence_after();
+      if (tracer) stamp_block(blk, 0);
       // (the scores waited for the products that last read this buffer, its dS^T tile among them)
       uint8_t* rowp = sdS + bf * kDsBytes + row * 128;
 #pragma unroll
@@ -1260,6 +1284,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_ld_cols(t_lane + col, rs);
         tmem_ld_cols(t_lane + col + 64, rp);
         tmem_ld_wait();
+        if (tracer && sub == 0) stamp_block(blk, 1);
         // Queries below the key row (causal) and key rows past the end have P = 0: their scaled scores become -inf. (A
         // second, masked copy of the block below ran twice an item, each time from a cold instruction cache, and took
         // 2000 cycles longer than the plain one.)
@@ -1268,7 +1293,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (__any_sync(0xffffffffu, (lim > 0) | past)) {
           const uint32_t live = (past || lim >= kCols) ? 0u : lim <= 0 ? 0xffffffffu : 0xffffffffu << lim;
 #pragma unroll
-          for (int i = 0; i < kCols; ++i) rs[i] = (live & (1u << i)) ? rs[i] : kPositive ? 0xff800000u : p.dead_score;
+          for (int i = 0; i < kCols; ++i) rs[i] = (live & (1u << i)) ? rs[i] : kPlain ? 0xff800000u : p.dead_score;
         }
         uint32_t pw[kCols];   // P^T as bf16 pairs, then dS^T
 #pragma unroll
@@ -1302,18 +1327,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.pds_full[bf]);
+      if (tracer) stamp_block(blk, 2);
+      blk += kGroups;
 #pragma unroll
       for (int i = 0; i < kGroups; ++i) {
         advance(cur);
         if (++bf == kBufs) { bf = 0; bph ^= 1; }
       }
     }
+    if (tracer && grp == 0) stamp(5);
   } else if (warp >= 4 + 8 * kGroups) {
     // ---------------- dQ drain warps: 32 values of head_dim (one per lane), 64 queries --------
     const int quad = warp & 3;
     const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
     float* stg = reinterpret_cast<float*>(sDQ + quad * 2 * kDqBytes);
-    uint32_t n = 0, bf = 0, bph = 0;
+    uint32_t n = 0, bf = 0, bph = 0, blk = 0;
     bool ok = true;
     for (int k = 0; k < rounds && ok; ++k) {
       const int w = item_at(k);
@@ -1325,6 +1353,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int qi = i0; qi < num_qb; ++qi) {
           if (!mbar_wait_warp(&ctl.dq_full[bf], bph, &abort_flag, p.status, kTimeoutTmemFull, 100)) { ok = false; break; }
           tc_fence_after();
+          if (quad == 0 && lane == 0) stamp_block(blk, 3);
           // 64 queries at once where registers allow it, so that the columns are handed back early
           constexpr int kAtOnce = (kGroups == 1) ? 2 : 1;
           uint32_t r[kAtOnce][32];
@@ -1354,6 +1383,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               bulk_commit_group();
             }
           }
+          if (quad == 0 && lane == 0) stamp_block(blk, 4);
+          ++blk;
           if (++bf == kBufs) { bf = 0; bph ^= 1; }
         }
       }
@@ -1372,6 +1403,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     __syncwarp();
     tmem_dealloc(tmem_base, kTmemCols);
   }
+  if (threadIdx.x == 0) stamp(6);
 }
 
 static long long* g_attn_trace = nullptr;
@@ -1519,8 +1551,8 @@ MMJ_API int mmj_attn_fwd(const void* q, long long ldq, int q_col0, const void* k
   return (int)cudaGetLastError();
 }
 
-// Install (or clear, with nullptr) the timeline buffer of the forward kernels: int64 [ctas * 64], written by whichever of
-// them is launched next. Launches whose grid has more CTAs than `ctas` leave it untouched.
+// Install (or clear, with nullptr) the timeline buffer of the attention kernels: int64
+// [ctas * 64], written by whichever of them is launched next. Launches whose grid has more CTAs than `ctas` leave it untouched.
 MMJ_API int mmj_attn_set_trace(void* buf, long long ctas) {
   g_attn_trace = reinterpret_cast<long long*>(buf);
   g_attn_trace_ctas = buf ? ctas : 0;
@@ -1582,11 +1614,12 @@ MMJ_API int mmj_attn_bwd(const void* q, long long ldq, int q_col0, const void* k
   // head_dim 128: 224 KB of tiles, the control block and the alignment padding take what is left of the 227 KB a CTA
   // may have (the kernel checks that they fit); head_dim 64 needs 208 KB of tiles
   const int smem = 232448;
+  p.trace = (g_attn_trace && (long long)grid.x <= g_attn_trace_ctas) ? g_attn_trace : nullptr;
   static bool attr_set[4] = {};
-  const bool positive = scale > 0.f;
-  auto* kernel = (D == 64) ? (positive ? &attn_bwd_kernel<64, true> : &attn_bwd_kernel<64, false>)
-                           : (positive ? &attn_bwd_kernel<128, true> : &attn_bwd_kernel<128, false>);
-  bool& attr = attr_set[(D == 64 ? 0 : 2) + (positive ? 1 : 0)];
+  const bool plain = scale > 0.f && p.trace == nullptr;
+  auto* kernel = (D == 64) ? (plain ? &attn_bwd_kernel<64, true> : &attn_bwd_kernel<64, false>)
+                           : (plain ? &attn_bwd_kernel<128, true> : &attn_bwd_kernel<128, false>);
+  bool& attr = attr_set[(D == 64 ? 0 : 2) + (plain ? 1 : 0)];
   if (!attr) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     attr = true;

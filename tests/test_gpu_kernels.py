@@ -402,6 +402,40 @@ def test_attention_backward_of_any_scale(T, D, scale):
             _close(a, e)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("backward", [False, True])
+def test_attention_timeline(D, backward):
+    """The clock stamps of forward and backward: taken in the order of the stages, results as without them."""
+    from momijo_b200 import _C
+
+    torch.manual_seed(13)
+    qkv, dy = _rand(512, 3 * D, grad=True), _rand(512, D)
+    run = lambda: ops.attention_packed(qkv, 1, 512, 1, 1, D)
+    y = run()
+    (plain,) = torch.autograd.grad(y, qkv, dy, retain_graph=True)
+    trace = torch.zeros(256, 64, dtype=torch.int64, device="cuda")
+    _C.call("mmj_attn_set_trace", trace.data_ptr(), 256)
+    try:
+        got = torch.autograd.grad(y, qkv, dy)[0] if backward else run()
+        torch.cuda.synchronize()
+    finally:
+        _C.call("mmj_attn_set_trace", None, 0)
+    if not backward:
+        assert torch.equal(got, y) and trace.any()
+        return
+    assert torch.equal(got[:, D:], plain[:, D:])    # (dQ adds up in the order of arrival)
+    _close(got[:, :D], plain[:, :D])
+    t = trace.cpu()
+    for cta in range(4):                            # four key blocks, the first one meets all eight query blocks
+        n = int(t[cta, 7])
+        assert n == 8 - 2 * cta and int(t[cta, 0]) < int(t[cta, 2]) < int(t[cta, 5]) < int(t[cta, 6])
+        for g in range(n):
+            seen, read, stored, dq, drained, issued = t[cta, 8 + 6 * g:14 + 6 * g].tolist()
+            assert 0 < seen < read < stored < issued < dq < drained
+        assert not t[cta, 8 + 6 * n:].any()
+    assert not t[4:].any()
+
+
 @pytest.mark.parametrize("B,T,Hq,Hkv,D", [(2, 37, 2, 1, 64), (1, 130, 4, 4, 128), (3, 5, 6, 2, 128)])
 def test_attention_rotary_paths(B, T, Hq, Hkv, D):
     """Rotation fused into the copy of the packed rows and into the gradient's cast, a misaligned input view among
