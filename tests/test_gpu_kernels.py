@@ -431,7 +431,7 @@ def test_attention_timeline(D, backward):
         assert n == 8 - 2 * cta and int(t[cta, 0]) < int(t[cta, 2]) < int(t[cta, 5]) < int(t[cta, 6])
         for g in range(n):
             seen, read, stored, dq, drained, issued = t[cta, 8 + 6 * g:14 + 6 * g].tolist()
-            assert 0 < seen < read < stored < issued < dq < drained
+            assert 0 < seen < read < stored and read < issued < dq < drained   # (a warp stamps after its arrival)
         assert not t[cta, 8 + 6 * n:].any()
     assert not t[4:].any()
 
