@@ -51,8 +51,8 @@ def pick_split(M: int, N: int, K: int) -> int:
     64 x 8192 x 4096 34.4 / 25.0 (1). With more tiles than that a second range finds no SM and pairs of CTAs win
     (1024 x 768 x 768 8.6 / 9.5), with a short contraction there is nothing to cut (64 x 64 x 64 4.3 / 5.9)."""
     tiles, blocks = -(-M // 128) * -(-N // 64), -(-K // 64)
-    if blocks < 8 or tiles > (148 if M < 256 else 64):
-        return 0
+    if blocks < 8 or tiles > (148 if M < 256 else 64) or (_PAIR["mode"] == "1" and M >= 256 and N >= 256):
+        return 0     # (mode 1: the pair kernel wherever it can run)
     s = 1
     while s < 8 and tiles * s * 2 <= 128 and blocks >= 4 * s:
         s *= 2

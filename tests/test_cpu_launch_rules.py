@@ -78,3 +78,13 @@ def test_split_rule_leaves_no_range_empty():
         for n in (8, 64, 72, 520, 2304):
             for k in (8, 64, 448, 512, 520, 576, 1024, 4096):
                 assert gemm_mod.pick_split(m, n, k) <= -(-k // 64)
+
+
+def test_pair_mode_one_takes_every_eligible_product(monkeypatch):
+    """MOMIJO_GEMM_PAIR=1 selects the pair kernel whenever it can run, ahead of the few-tile rule as well."""
+    monkeypatch.setitem(gemm_mod._PAIR, "mode", "1")
+    for m, n, k in ((256, 256, 512), (512, 512, 4096), (700, 640, 2000), (4096, 4096, 28672)):
+        assert gemm_mod.pick_split(m, n, k) == 0 and gemm_mod.pick_pair(m, n, k)
+    assert gemm_mod.pick_split(255, 512, 1024) > 0      # fewer than 256 rows: not eligible
+    monkeypatch.setitem(gemm_mod._PAIR, "mode", "auto")
+    assert gemm_mod.pick_split(512, 512, 4096) > 0
