@@ -89,6 +89,8 @@ def _weight_grad(x, dy, w, geom):
     n = _C.lib().mmj_conv2d_dw_scratch(geom)
     scratch = torch.empty(n, dtype=torch.float32, device=x.device) if n else None
     _C.call("mmj_conv2d_dw", _C.ptr(x), _C.ptr(dy), _C.ptr(dw), _C.ptr(scratch), geom, _dt(x), _C.current_stream())
+    if n:
+        _C.launches += 1     # slabs are folded by a second kernel
     return dw
 
 

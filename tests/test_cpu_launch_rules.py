@@ -88,3 +88,15 @@ def test_pair_mode_one_takes_every_eligible_product(monkeypatch):
     assert gemm_mod.pick_split(255, 512, 1024) > 0      # fewer than 256 rows: not eligible
     monkeypatch.setitem(gemm_mod._PAIR, "mode", "auto")
     assert gemm_mod.pick_split(512, 512, 4096) > 0
+
+
+@pytest.mark.parametrize("n,c,hw,oc,groups,kernels", [(32, 64, 56, 64, 1, 2), (4, 16, 20, 16, 16, 1)])
+def test_weight_gradient_counts_its_launches(monkeypatch, n, c, hw, oc, groups, kernels):
+    """Slices and their fold are two kernels, the direct form (depthwise here) is one."""
+    monkeypatch.setitem(_C._FNS, "mmj_conv2d_dw", (lambda *args: 0, _C._SIGS["mmj_conv2d_dw"][1]))
+    monkeypatch.setattr(_C, "current_stream", lambda: 0)
+    x, w = torch.zeros(n, c, hw, hw), torch.zeros(oc, c // groups, 3, 3)
+    geom = conv._geom(n, c, hw, hw, oc, 3, 3, hw, hw, (1, 1), (1, 1), (1, 1), groups)
+    before = _C.launches
+    conv._weight_grad(x, torch.zeros(n, oc, hw, hw), w, geom)
+    assert _C.launches - before == kernels
