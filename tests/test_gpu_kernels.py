@@ -436,7 +436,8 @@ def test_attention_timeline(D, backward):
     assert not t[4:].any()
 
 
-@pytest.mark.parametrize("B,T,Hq,Hkv,D", [(2, 37, 2, 1, 64), (1, 130, 4, 4, 128), (3, 5, 6, 2, 128)])
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [(2, 37, 2, 1, 64), (1, 130, 4, 4, 128), (3, 5, 6, 2, 128),
+                                           (1, 64, 1, 1, 64), (2, 32, 32, 8, 128)])
 def test_attention_rotary_paths(B, T, Hq, Hkv, D):
     """Rotation fused into the copy of the packed rows and into the gradient's cast, a misaligned input view among
     them, against the differentiable rotation of the CPU path."""
