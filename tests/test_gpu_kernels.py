@@ -384,22 +384,28 @@ def test_attention_backward_block_edges(B, T, Hq, Hkv, D, causal):
 @pytest.mark.parametrize("scale", [0.0, -0.1, 0.3])
 @pytest.mark.parametrize("T,D", [(64, 64), (192, 64), (192, 128), (256, 128)])
 def test_attention_backward_of_any_scale(T, D, scale):
-    """Key rows past the end of the last key block take no part, whatever the sign of the scale (0: equal weights)."""
+    """Key rows past the end of the last key block take no part, whatever the sign of the scale (0: equal weights). The
+    launcher is given the forward's results in 64 bits, rounded as the forward kernel stores them."""
+    from momijo_b200 import _C
+
     torch.manual_seed(12)
-    qkv, dy = _rand(2 * T, 4 * D, grad=True), _rand(2 * T, 2 * D)
-    y = ops.attention_packed(qkv, 2, T, 2, 1, D, causal=False, scale=scale)
-    (got,) = torch.autograd.grad(y, qkv, dy)
-    x = qkv.detach().double().cpu().requires_grad_()
+    qkv, dy, ld = _rand(2 * T, 4 * D), _rand(2 * T, 2 * D), 4 * D
+    x = qkv.double().cpu().requires_grad_()
     v = x.view(2, T, 4, D).transpose(1, 2)
-    p = torch.softmax(v[:, :2] @ v[:, 2:3].transpose(-1, -2) * scale, -1)
-    ref = (p @ v[:, 3:]).transpose(1, 2).reshape(2 * T, 2 * D)
+    s = v[:, :2] @ v[:, 2:3].transpose(-1, -2) * scale
+    ref = (torch.softmax(s, -1) @ v[:, 3:]).transpose(1, 2).reshape(2 * T, 2 * D)
     (want,) = torch.autograd.grad(ref, x, dy.double().cpu())
-    _close(y, ref.detach().cuda())
-    for lo, hi in ((0, 2), (2, 3), (3, 4)):
-        a, e = got[:, lo * D:hi * D], want[:, lo * D:hi * D].cuda()
-        assert not a.any() if scale == 0.0 and lo < 3 else True     # dQ and dK carry the scale as a factor
-        if scale != 0.0 or lo == 3:
-            _close(a, e)
+    out, lse = ref.detach().to(bf16).cuda(), torch.logsumexp(s, -1).detach().float().cuda().contiguous()
+    delta, dq, got = torch.empty_like(lse), torch.empty(2 * T, 2 * D, device="cuda"), torch.empty_like(qkv)
+    _C.call("mmj_attn_bwd", qkv.data_ptr(), ld, 0, qkv.data_ptr(), ld, 2 * D, qkv.data_ptr(), ld, 3 * D, out.data_ptr(),
+            2 * D, 0, dy.data_ptr(), 2 * D, 0, lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), 2 * D, 0, got.data_ptr(), ld,
+            2 * D, got.data_ptr(), ld, 3 * D, 2, T, 2, 1, D, scale, 0, _C.status_tensor(qkv.device).data_ptr(),
+            _C.current_stream())
+    for a, e in ((dq, want[:, :2 * D]), (got[:, 2 * D:3 * D], want[:, 2 * D:3 * D]), (got[:, 3 * D:], want[:, 3 * D:])):
+        if e.any():
+            _close(a, e.cuda())
+        else:
+            assert not a.any()      # scale 0 is a factor of dQ and dK
 
 
 @pytest.mark.parametrize("D", [64, 128])
