@@ -634,56 +634,56 @@ __global__ void __launch_bounds__(kWgThreads, 4)
 }
 
 // The tiles multiply pixels outside the image as zeros, which an infinite dy turns into NaN where the tap does not exist:
-// a NaN sum of one slice [pb, pe) again without such pixels, in chains of 64 as well. i: (filter, channel, tap).
+// a NaN sum again without such pixels, in chains of 64 and slices as well. i: (filter, channel, tap).
 template <typename T>
-__device__ __noinline__ float wgrad_skip_sum(const T* x, const T* dy, const ConvGeom& g, long long i, long long pb,
-                                             long long pe, float nan) {
+__device__ __noinline__ void wgrad_skip_sum(const T* x, const T* dy, T* dst, const ConvGeom& g, long long i,
+                                            long long slice) {
   const int cg = g.C / g.groups, taps = g.kH * g.kW, K = cg * taps, spatial = g.OH * g.OW;
   const int oc = (int)(i / K), k = (int)(i - (long long)oc * K), ch = k / taps, t = k - ch * taps;
   const int eh = t / g.kW * g.dh - g.ph, ew = t % g.kW * g.dw - g.pw;
-  if (eh >= 0 && (g.OH - 1) * g.sh + eh < g.H && ew >= 0 && (g.OW - 1) * g.sw + ew < g.W) return nan;   // never outside
+  if (eh >= 0 && (g.OH - 1) * g.sh + eh < g.H && ew >= 0 && (g.OW - 1) * g.sw + ew < g.W) return;   // never outside
   const T* xc = x + (long long)(oc / (g.OC / g.groups) * cg + ch) * g.H * g.W;
-  float total = 0.f, part = 0.f;
-  for (long long p = pb; p < pe; ++p) {
+  float all = 0.f, total = 0.f, part = 0.f;
+  const long long P = (long long)g.N * spatial;
+  for (long long p = 0; p < P; ++p) {
     const int n = (int)(p / spatial), s = (int)(p - (long long)n * spatial);
     const int h = s / g.OW * g.sh + eh, w = s % g.OW * g.sw + ew;
     if ((unsigned)h < (unsigned)g.H && (unsigned)w < (unsigned)g.W)
       part = fmaf(to_f<T>(dy[((long long)n * g.OC + oc) * spatial + s]),
                   to_f<T>(xc[(long long)n * g.C * g.H * g.W + (long long)h * g.W + w]), part);
-    if (((p - pb) & 63) == 63) {
+    if ((p & 63) == 63) {
       total += part;
       part = 0.f;
     }
+    if ((p + 1) % slice == 0) {
+      all += total + part;
+      total = part = 0.f;
+    }
   }
-  return total + part;
+  dst[i] = from_f<T>(all + total + part);
 }
 
 // dst[i] = sum over S slabs: 8 lanes of slabs per element group, folded in a fixed order. kConv: slabs of a weight
-// gradient over slices of `slice` positions.
+// gradient over slices of `slice` positions; its NaNs are looked at last, in 32 registers, so that they cost the fold
+// neither registers nor blocks (a call among its loads took 1 x 4096 channels, 1000 filters from 150 to 359 us).
 template <typename T, bool kConv>
-__global__ void __launch_bounds__(256) slab_fold_kernel(const float* __restrict__ slabs, T* __restrict__ dst, long long n,
-                                                        int S, const T* __restrict__ x, const T* __restrict__ dy,
-                                                        const __grid_constant__ ConvGeom g, long long slice) {
+__global__ void __launch_bounds__(256, 8) slab_fold_kernel(const float* __restrict__ slabs, T* __restrict__ dst,
+                                                           long long n, int S, const T* __restrict__ x,
+                                                           const T* __restrict__ dy, const __grid_constant__ ConvGeom g,
+                                                           long long slice) {
   __shared__ float part[8][32];
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
   const long long i = (long long)blockIdx.x * 32 + lane;
   float a = 0.f;
   if (i < n)
-    for (int s = row; s < S; s += 8) {
-      float v = slabs[(long long)s * n + i];
-      if (kConv && v != v) {
-        const long long pb = s * slice, P = (long long)g.N * g.OH * g.OW;
-        v = wgrad_skip_sum<T>(x, dy, g, i, pb, pb + slice < P ? pb + slice : P, v);
-      }
-      a += v;
-    }
+    for (int s = row; s < S; s += 8) a += slabs[(long long)s * n + i];
   part[row][lane] = a;
   __syncthreads();
-  if (row == 0 && i < n) {
+  if (row != 0 || i >= n) return;
 #pragma unroll
-    for (int r = 1; r < 8; ++r) a += part[r][lane];
-    dst[i] = from_f<T>(a);
-  }
+  for (int r = 1; r < 8; ++r) a += part[r][lane];
+  dst[i] = from_f<T>(a);
+  if (kConv && a != a) wgrad_skip_sum<T>(x, dy, dst, g, i, slice);
 }
 
 // db[oc] = sum_{n, oh, ow} dy[n, oc, oh, ow]: `splits` blocks per channel over whole images (one block per channel
