@@ -84,8 +84,8 @@ _SIGS = {
     "mmj_conv2d_dx": ([P, P, P, P, P, I, P], 1),
     "mmj_conv2d_dw": ([P, P, P, P, P, I, P], 1),
     "mmj_conv2d_dw_scratch": ([P], 0),
-    "mmj_channel_sum": ([P, P, P, I, I, L, I, P], 2),
-    "mmj_channel_sum_splits": ([I, I], 0),
+    "mmj_channel_sum": ([P, P, P, I, I, L, I, P], 1),
+    "mmj_channel_sum_splits": ([I, I, L], 0),
     "mmj_maxpool2d_fwd": ([P, P, P, P, I, P], 1),
     "mmj_maxpool2d_bwd": ([P, P, P, P, I, P], 1),
     "mmj_avgpool2d_fwd": ([P, P, P, I, P], 1),

@@ -97,8 +97,11 @@ def _weight_grad(x, dy, w, geom):
 def _channel_sum(dy, N, C, spatial):
     """Sums of a [N, C, spatial] tensor over images and positions (bias gradient)."""
     db = torch.empty(C, dtype=dy.dtype, device=dy.device)
-    scratch = torch.empty(_C.lib().mmj_channel_sum_splits(N, C) * C, dtype=torch.float32, device=dy.device)
+    S = _C.lib().mmj_channel_sum_splits(N, C, spatial)
+    scratch = torch.empty(S * C, dtype=torch.float32, device=dy.device) if S > 1 else None
     _C.call("mmj_channel_sum", _C.ptr(dy), _C.ptr(db), _C.ptr(scratch), N, C, spatial, _dt(dy), _C.current_stream())
+    if S > 1:
+        _C.launches += 1     # the blocks' sums are folded by a second kernel
     return db
 
 

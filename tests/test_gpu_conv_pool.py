@@ -202,3 +202,16 @@ def test_infinite_values_meet_only_taps_inside_the_image(dtype, H, s, p, d):
             # sums of up to n products: 4 * 2^-24 * sqrt(n) of the norm, and 2^-8 for a bf16 result
             tol = 4 * 2.0 ** -24 * (N * OH * OH) ** 0.5 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
             assert float((a - e)[fin].norm()) <= tol * float(e[fin].norm())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,C,spatial", [(1, 1, 1), (257, 8, 1), (300, 3, 7), (5, 300, 33), (3, 5, 257), (9, 2, 2049),
+                                         (40, 2, 1024), (2, 64, 9000)])
+def test_channel_sums(dtype, N, C, spatial):
+    """Fewer positions than threads and more, one block to a channel and several, against 64 bits."""
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    dy = torch.randn(N, C, spatial, generator=gen, device="cuda").to(dtype)
+    got, want = cv._channel_sum(dy, N, C, spatial).double(), dy.double().sum((0, 2))
+    # chains of at most a few hundred additions, of sums no larger than the values' own sum
+    tol = 2.0 ** -24 * 32 * dy.double().abs().sum((0, 2)) + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
+    assert ((got - want).abs() <= tol).all()
