@@ -981,6 +981,12 @@ static int wgrad_slices(const ConvGeom& g, long long* slice) {
   const long long tiles_m = (long long)((ocg + bm - 1) / bm) * g.groups, tiles_k = (K + kWgBN - 1) / kWgBN;
   // fewer than 8 filter taps in a 64-wide tile is mostly padding
   if (!tiled_ok(g, ocg) || K < 8 || tiles_m > 65535 || P > 0x7fffff00LL) return 0;
+  // A small gradient stays with the direct kernel, one block to an element: the tiles' chain and the fold take 11 to 14 us
+  // at least, the direct blocks about 2.4 us a thousand positions (of 1000 and more) and 500 elements. Direct / tiled, us:
+  // one filter of 9 weights, 196 positions 2.4 / 11.2, 3136 8.9 / 14.1, 12544 29.3 / 13.3; 3 x 121 weights, 3136 positions
+  // 12.0 / 14.1; 64 x 9 14.8 / 14.0; 64 x 25, 784 positions 14.7 / 13.8; 8 x 576, 12544 positions 315 / 19.
+  const long long elems = g.OC * K, pos = P > 1000 ? P : 1000;
+  if (pos * (elems > 500 ? elems : 500) < 3700 * 500) return 0;
   long long s = (2 * 4 * 148 + tiles_m * tiles_k - 1) / (tiles_m * tiles_k);
   const long long by_work = P / 256, by_mem = (64LL << 20) / (4 * g.OC * K);
   if (s > by_work) s = by_work;

@@ -100,3 +100,12 @@ def test_weight_gradient_counts_its_launches(monkeypatch, n, c, hw, oc, groups, 
     before = _C.launches
     conv._weight_grad(x, torch.zeros(n, oc, hw, hw), w, geom)
     assert _C.launches - before == kernels
+
+
+@pytest.mark.parametrize("n,c,hw,oc,k,direct", [
+    (1, 32, 14, 4, 1, True), (1, 1, 56, 1, 3, True), (16, 3, 14, 1, 11, True),     # fewer positions or weights than pay
+    (4, 1, 56, 1, 3, False), (4, 64, 14, 64, 3, False), (1, 512, 7, 512, 3, False)])
+def test_small_weight_gradients_stay_direct(n, c, hw, oc, k, direct):
+    """No slabs are asked for where one block to a weight is the faster form."""
+    geom = conv._geom(n, c, hw, hw, oc, k, k, hw, hw, (1, 1), (k // 2, k // 2), (1, 1), 1)
+    assert (_C.lib().mmj_conv2d_dw_scratch(geom) == 0) == direct
