@@ -399,7 +399,9 @@ __global__ void __launch_bounds__(kGatherThreads, 3)
       tab[c % 3][t] = e;
     }
   };
-  float ra[LA], rb[BK];
+  // widened when they are staged: here the conversion waits for its load before the products of this chunk (bf16,
+  // N4 C64 28x28, 8 filters, k11: 489 us, 334 now)
+  T ra[LA], rb[BK];
   auto fetch = [&](int c) {
     const int4* tb = tab[c % 3];
 #pragma unroll
@@ -407,23 +409,23 @@ __global__ void __launch_bounds__(kGatherThreads, 3)
       const int id = t + i * kGatherThreads;
       const int kk = id % BK, m = id / BK;
       const int off = tb[kk].w;
-      ra[i] = (off >= 0 && m0 + m < g.M) ? to_f<T>(wp[(long long)m * g.w_m + off]) : 0.f;
+      ra[i] = (off >= 0 && m0 + m < g.M) ? wp[(long long)m * g.w_m + off] : from_f<T>(0.f);
     }
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       const int4 e = tb[kk];
       const bool ok = ((unsigned)(h0 + e.y) < (unsigned)g.SH) & ((unsigned)(w0 + e.z) < (unsigned)g.SW);
-      rb[kk] = ok ? to_f<T>(sp[e.x]) : 0.f;
+      rb[kk] = ok ? sp[e.x] : from_f<T>(0.f);
     }
   };
   auto stage = [&](int buf) {
 #pragma unroll
     for (int i = 0; i < LA; ++i) {
       const int id = t + i * kGatherThreads;
-      As[buf][id % BK][id / BK] = ra[i];
+      As[buf][id % BK][id / BK] = to_f<T>(ra[i]);
     }
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) Bs[buf][kk][t] = rb[kk];
+    for (int kk = 0; kk < BK; ++kk) Bs[buf][kk][t] = to_f<T>(rb[kk]);
   };
 
   f32x2 acc[TM][TN / 2];
@@ -529,7 +531,7 @@ __global__ void __launch_bounds__(kWgThreads, 4)
   }
   const T* xg = x + (long long)grp * cg * g.H * g.W;
   const T* yg = dy + ((long long)grp * ocg + m0) * spatial;
-  float ra[RA], rb[RB];
+  T ra[RA], rb[RB];
   auto fetch = [&](long long p) {
     p += lane;
     int h0 = -(1 << 29), w0 = 0;
@@ -547,22 +549,24 @@ __global__ void __launch_bounds__(kWgThreads, 4)
 #pragma unroll
     for (int i = 0; i < RA; ++i) {
       const int m = warp * RA + i;
-      ra[i] = (live && m0 + m < ocg) ? to_f<T>(yp[(long long)m * spatial]) : 0.f;
+      ra[i] = (live && m0 + m < ocg) ? yp[(long long)m * spatial] : from_f<T>(0.f);
     }
 #pragma unroll
     for (int i = 0; i < RB; ++i) {
       const int4 e = tab[warp * RB + i];
       const bool ok = ((unsigned)(h0 + e.y) < (unsigned)g.H) & ((unsigned)(w0 + e.z) < (unsigned)g.W);
-      rb[i] = ok ? to_f<T>(sp[e.x]) : 0.f;
+      rb[i] = ok ? sp[e.x] : from_f<T>(0.f);
     }
   };
   auto stage = [&](int buf) {
 #pragma unroll
     for (int i = 0; i < RA; i += 4)
-      *reinterpret_cast<float4*>(&As[buf][lane][warp * RA + i]) = make_float4(ra[i], ra[i + 1], ra[i + 2], ra[i + 3]);
+      *reinterpret_cast<float4*>(&As[buf][lane][warp * RA + i]) =
+          make_float4(to_f<T>(ra[i]), to_f<T>(ra[i + 1]), to_f<T>(ra[i + 2]), to_f<T>(ra[i + 3]));
 #pragma unroll
     for (int i = 0; i < RB; i += 4)
-      *reinterpret_cast<float4*>(&Bs[buf][lane][warp * RB + i]) = make_float4(rb[i], rb[i + 1], rb[i + 2], rb[i + 3]);
+      *reinterpret_cast<float4*>(&Bs[buf][lane][warp * RB + i]) =
+          make_float4(to_f<T>(rb[i]), to_f<T>(rb[i + 1]), to_f<T>(rb[i + 2]), to_f<T>(rb[i + 3]));
   };
   f32x2 acc[TM][TN / 2];
   float sum[TM][TN];
