@@ -892,14 +892,28 @@ MMJ_API int mmj_col2im(const void* cols, void* dx, const int* geom, long long ld
 // The tiled kernels address one image and one filter bank with 32-bit offsets. Their narrowest tile has 16 output
 // channels, so a depthwise layer fills one row of it and stays with the one-thread-per-output kernels (N32 C64
 // 56x56 k3, direct / tiled, us: forward 128 / 230, input gradient 223 / 343, weight gradient 361 / 853). From two
-// channels per group the tiles win (32 groups of 2: 190 / 180, 386 / 235, 685 / 368), and without groups even a
-// single filter does (N16 C64 56x56 OC1: forward 88 / 55, weight gradient 182 / 62).
+// channels per group the tiles win (32 groups of 2: 190 / 180, 386 / 235, 685 / 368), and without groups a single
+// filter mostly does (N16 C64 56x56 OC1: forward 88 / 55, weight gradient 182 / 62; see lone_channel_direct).
 static inline bool tiled_ok(const ConvGeom& g, int m_per_group) {
   const long long lim = 0x3fffffffLL;
   return (m_per_group >= 2 || g.groups == 1) && (long long)g.C * g.H * g.W < lim && (long long)g.OC * g.OH * g.OW < lim &&
          (long long)g.OC * (g.C / g.groups) * g.kH * g.kW < lim && (long long)g.kH * g.dh * g.W < lim &&
          (long long)g.H + g.ph + (long long)g.kH * g.dh < (1 << 28) &&
          (long long)g.W + g.pw + (long long)g.kW * g.dw < (1 << 28);
+}
+// One output channel without groups: the tiles win by their blocks in flight, until the positions alone give the direct
+// kernel enough of them and long rows of taps read the image from cache. fp32, direct / tiled, us: forward of 200704
+// positions, 3x3 taps of 1 / 3 / 8 / 32 channels 6.8 / 9.1, 12.1 / 13.6, 24.8 / 25.5, 85.7 / 79.3, 5x5 of 1 / 64 channels
+// 8.7 / 13.3, 303 / 420; of 65536 positions 3x3 of 1 channel 3.4 / 4.1; of 50176 3x3 of 8 12.2 / 8.6, 5x5 of 1 / 64 4.4 / 4.9, 136 / 126, 11x11 of 64
+// 483 / 593; of 12544 positions 11x11 of 64 453 / 332. The input gradient's direct kernel checks every tap against the
+// stride: 200704 positions, 3x3 taps of 1 / 3 filters 10.5 / 12.1, 24.0 / 16.4.
+static inline bool lone_channel_direct(const GatherGeom& t) {
+  if (t.M != 1 || t.cls_h != 1 || t.cls_w != 1) return false;
+  const long long P = (long long)t.N * t.PHf * t.PWf;
+  const int taps = t.kH * t.kW;
+  if (t.transposed) return P >= 768 * 148 && taps >= 9 && t.channels * taps <= 9;
+  return (P >= 768 * 148 && (taps >= 25 || (taps >= 9 && t.channels <= 8))) ||
+         (P >= 256 * 148 && (taps >= 81 || (taps >= 25 && t.channels <= 8) || (taps >= 9 && t.channels == 1)));
 }
 // 64-channel tiles unless they would leave a half-empty last one
 static inline int tile_rows(int m) { return m <= 16 ? 16 : (m % 64 >= 1 && m % 64 <= 32) ? 32 : 64; }
@@ -939,7 +953,7 @@ MMJ_API int mmj_conv2d_fwd(const void* x, const void* w, const void* bias, void*
   t.src_n = (long long)g.C * g.H * g.W; t.src_g = (long long)cg * g.H * g.W;
   t.w_ch = (long long)g.kH * g.kW; t.w_m = t.w_ch * cg; t.w_g = t.w_m * ocg;
   t.dst_m = (long long)g.OH * g.OW; t.dst_g = t.dst_m * ocg; t.dst_n = t.dst_m * g.OC;
-  if (tiled_ok(g, ocg) && grid_fits(t)) {
+  if (tiled_ok(g, ocg) && grid_fits(t) && !lone_channel_direct(t)) {
     DISPATCH(dtype, return launch_gather<float>(x, w, bias, y, t, STREAM),
              return launch_gather<__nv_bfloat16>(x, w, bias, y, t, STREAM));
   }
@@ -964,7 +978,7 @@ MMJ_API int mmj_conv2d_dx(const void* dy, const void* w, const void* bias, void*
   t.w_m = (long long)g.kH * g.kW; t.w_ch = t.w_m * cg; t.w_g = t.w_ch * ocg;
   t.dst_m = (long long)g.H * g.W; t.dst_g = t.dst_m * cg; t.dst_n = t.dst_m * g.C;
   // a stride larger than the image would leave classes without pixels
-  if (tiled_ok(g, cg) && grid_fits(t) && g.sh <= g.H && g.sw <= g.W) {
+  if (tiled_ok(g, cg) && grid_fits(t) && g.sh <= g.H && g.sw <= g.W && !lone_channel_direct(t)) {
     DISPATCH(dtype, return launch_gather<float>(dy, w, bias, dx, t, STREAM),
              return launch_gather<__nv_bfloat16>(dy, w, bias, dx, t, STREAM));
   }
