@@ -78,10 +78,22 @@ def col2im(cols, x_shape, kernel, stride=(1, 1), pad=(0, 0), dilation=(1, 1)):
 
 
 # ---- convolution ----------------------------------------------------------------------------------------
-# bf16 input gradients up to this many filters come from the direct kernel, whose time grows with them, and above from a
-# product and its overlapping sums. Direct / product and sums, us, k3: N32 C64 56x56 16 filters 83 / 282, 32 143 / 290,
-# N32 C128 28x28 48 103 / 155; at 64 filters it depends on the shape (265 / 303, N8 C32 30x30 k5 135 / 85), at 128 511 / 333.
-_DIRECT_DX_CHANNELS = 48
+def _direct_dx(N, C, H, W, OC, OH, OW, taps, classes):
+    """Whether a bf16 input gradient comes from the direct kernel or from a product and its overlapping sums. Both times
+    in us, fitted to 3954 shapes (C 3 to 512, OC 16 to 96, 7x7 to 56x56, N 1 to 32, k 1 to 5, stride 1 and 2; rms error
+    14 and 18 %): the direct kernel by its chain of 16-deep chunks and its multiply-adds, padding of its tiles
+    included, the product by the patch matrix, the sums' reads and dy. The margin leaves 0.5 % of the shapes more than
+    5 % slower than with the product, by 1.18 at most. Direct / product, k3: N32 C64 56x56 16 filters 83 / 282, 32 143 / 290, N1 C512
+    14x14 48 filters 33 / 22; k5: N1 C32 14x14 48 filters 61 / 19; k11: N4 C1 224x224 32 filters 1039 / 156."""
+    P = N * -(-H * W // classes)
+    bm = 16 if C <= 16 else 32 if 1 <= C % 64 <= 32 else 64         # as the launcher chooses it
+    blocks = lambda rows: -(-P // 128) * -(-C // rows) * classes
+    while bm > 16 and blocks(bm) < 148:
+        bm //= 2
+    K = OC * taps / classes
+    direct = 7.4 + 0.66 * K / 16 + 55e-9 * blocks(bm) * 128 * bm * K
+    product = 14.0 + 1e-6 * (1.5 * N * OH * OW * C * taps + 2.3 * N * C * H * W * taps + 6.5 * N * OH * OW * OC)
+    return direct < 0.85 * product
 
 
 def _weight_grad(x, dy, w, geom):
@@ -153,7 +165,7 @@ class _Conv2d(torch.autograd.Function):
             if Kp != K:
                 w2 = tF.pad(w2, (0, Kp - K))
             if ctx.needs_input_grad[0]:
-                if OC <= _DIRECT_DX_CHANNELS:
+                if _direct_dx(N, C, H, W, OC, OH, OW, kH * kW, stride[0] * stride[1]):
                     dx = torch.empty_like(x)
                     _C.call("mmj_conv2d_dx", _C.ptr(dy), _C.ptr(w), None, _C.ptr(dx), ctx.geom, _dt(x),
                             _C.current_stream())

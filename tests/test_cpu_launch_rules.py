@@ -109,3 +109,13 @@ def test_small_weight_gradients_stay_direct(n, c, hw, oc, k, direct):
     """No slabs are asked for where one block to a weight is the faster form."""
     geom = conv._geom(n, c, hw, hw, oc, k, k, hw, hw, (1, 1), (k // 2, k // 2), (1, 1), 1)
     assert (_C.lib().mmj_conv2d_dw_scratch(geom) == 0) == direct
+
+
+@pytest.mark.parametrize("n,c,hw,oc,k,stride,direct", [
+    (32, 64, 56, 16, 3, 1, True), (32, 64, 56, 32, 3, 1, True), (32, 64, 56, 64, 1, 1, True),
+    (1, 512, 14, 48, 3, 1, False), (2, 48, 20, 48, 3, 1, False), (1, 32, 14, 48, 5, 1, False),   # few positions
+    (4, 1, 224, 32, 11, 1, False), (16, 3, 56, 32, 5, 1, False),                                # rows of padding
+    (32, 64, 56, 128, 3, 1, False)])
+def test_bf16_input_gradient_takes_the_faster_route(n, c, hw, oc, k, stride, direct):
+    o = (hw + 2 * (k // 2) - k) // stride + 1
+    assert conv._direct_dx(n, c, hw, hw, oc, o, o, k * k, stride * stride) == direct

@@ -135,10 +135,12 @@ def test_conv2d_tile_edges_against_64_bits(N, C, H, W, OC, k, s, p, d, g):
 
 @pytest.mark.parametrize("N,C,H,W,OC,k,s,p,d", [(2, 7, 9, 11, 16, 3, 1, 1, 1), (1, 16, 13, 8, 56, 3, 2, 1, 1),
                                                 (2, 24, 10, 10, 72, (3, 1), 1, 1, 2), (1, 64, 33, 5, 48, 1, 1, 0, 1),
-                                                (1, 16, 13, 8, 49, 3, 2, 1, 1), (2, 9, 7, 10, 17, 3, 1, 1, 1)])
-def test_bf16_lowered_convolution(N, C, H, W, OC, k, s, p, d):
-    """The patch matrix (exact: it only moves values) and both ways of the input gradient, on either side of the filter
-    count where they change; results rounded to bf16. The product takes filters in eights only: 49 and 17 stay direct."""
+                                                (1, 16, 13, 8, 49, 3, 2, 1, 1), (2, 9, 7, 10, 17, 3, 1, 1, 1),
+                                                (4, 24, 55, 57, 16, 3, 1, 1, 1)])     # patches of 64 columns to a warp
+@pytest.mark.parametrize("direct_dx", [False, True])
+def test_bf16_lowered_convolution(monkeypatch, direct_dx, N, C, H, W, OC, k, s, p, d):
+    """The patch matrix (exact: it only moves values) and both ways of the input gradient; results rounded to bf16. The product takes filters in eights only: 49 and 17 stay direct."""
+    monkeypatch.setattr(cv, "_direct_dx", lambda *shape: direct_dx)
     kh, kw = (k, k) if isinstance(k, int) else k
     gen = torch.Generator(device="cuda").manual_seed(4)
     r = lambda *shape: torch.randn(*shape, generator=gen, device="cuda").bfloat16()
