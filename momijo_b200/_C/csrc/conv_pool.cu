@@ -29,25 +29,43 @@ template <> __device__ __forceinline__ float from_f<float>(float v) { return v; 
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16(v); }
 
 // ---- im2col: cols[(n, oh, ow), c * kH * kW + kh * kW + kw], row pitch ldc >= C*kH*kW (pad columns = 0) ----
-// A warp owns 32 output positions and 64 columns: it gathers with the positions along its lanes (contiguous in the image
-// rows, one tap for the whole warp, stepped without divisions), turns the tile through shared memory and stores rows of
-// 64 columns. One element per thread, consecutive threads along a row of cols, took two 64-bit divisions each and
-// gathered 32 sectors with every load: 504 us for 100352 x 576 bf16, 82 now.
+// Small matrices (up to 131072 elements), an element to a thread: 49 x 72 bf16 in 1.5 us, where the kernel below has a
+// chain of gathers and stores (2.9 with 16 columns to a warp, 5.1 with 64).
 template <typename T>
+__global__ void __launch_bounds__(256) im2col_small_kernel(const T* __restrict__ x, T* __restrict__ cols, ConvGeom g, int ldc) {
+  const int i = blockIdx.x * 256 + threadIdx.x, r = i / ldc, k = i - r * ldc;
+  if (r >= g.N * g.OH * g.OW) return;
+  T v = from_f<T>(0.f);
+  if (k < g.C * g.kH * g.kW) {
+    const int t = k / g.kW, kw = k - t * g.kW, c = t / g.kH, kh = t - c * g.kH;
+    const int q = r / g.OW, ow = r - q * g.OW, n = q / g.OH, oh = q - n * g.OH;
+    const int h = oh * g.sh - g.ph + kh * g.dh, w = ow * g.sw - g.pw + kw * g.dw;
+    if (h >= 0 && h < g.H && w >= 0 && w < g.W) v = x[(((long long)n * g.C + c) * g.H + h) * g.W + w];
+  }
+  cols[i] = v;
+}
+
+// A warp owns 32 output positions and KT columns: it gathers with the positions along its lanes (contiguous in the image
+// rows, one tap for the whole warp, stepped without divisions), turns the tile through shared memory and stores rows of
+// KT columns. One element per thread, consecutive threads along a row of cols, took two 64-bit divisions each and
+// gathered 32 sectors with every load: 504 us for 100352 x 576 bf16, 82 now with 64 columns. Smaller matrices have too few
+// warps of 64 columns, whose gathers follow one another: 3136 x 144 in 7.0 us with an element per thread, 5.4 with 64
+// columns to a warp, 3.6 with 16; 25088 x 64 17.5 / 6.5 / 5.4.
+template <typename T, int KT>
 __global__ void __launch_bounds__(128) im2col_kernel(const T* __restrict__ x, T* __restrict__ cols, ConvGeom g,
                                                      long long ldc, int vec) {
   constexpr int V = 16 / sizeof(T);             // elements per 16-byte store
-  constexpr int kPitch = 64 + V;                // rows stay 16-byte aligned
+  constexpr int kPitch = KT + V;                // rows stay 16-byte aligned
   __shared__ __align__(16) T tile[4][32 * kPitch];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   T* st = tile[warp];
   const long long rows = (long long)g.N * g.OH * g.OW;
   const int K = g.C * g.kH * g.kW;
-  const int k_tiles = (int)((ldc + 63) / 64);
+  const int k_tiles = (int)((ldc + KT - 1) / KT);
   const long long units = (rows + 31) / 32 * k_tiles;
   for (long long u = blockIdx.x * 4LL + warp; u < units; u += gridDim.x * 4LL) {
     const long long r0 = u / k_tiles * 32;
-    const int k0 = (int)(u % k_tiles) * 64;
+    const int k0 = (int)(u % k_tiles) * KT;
     const long long r = r0 + lane;
     int h0 = -(1 << 29), w0 = 0;                // a position past the end reads nothing
     const T* xp = x;
@@ -62,7 +80,7 @@ __global__ void __launch_bounds__(128) im2col_kernel(const T* __restrict__ x, T*
     int c = k0 / (g.kH * g.kW), t = k0 - c * g.kH * g.kW;
     int kh = t / g.kW, kw = t - kh * g.kW;
 #pragma unroll 8
-    for (int j = 0; j < 64; ++j) {
+    for (int j = 0; j < KT; ++j) {
       const int dh = kh * g.dh, dw = kw * g.dw;
       T v = from_f<T>(0.f);
       if (k0 + j < K && (unsigned)(h0 + dh) < (unsigned)g.H && (unsigned)(w0 + dw) < (unsigned)g.W)
@@ -74,17 +92,17 @@ __global__ void __launch_bounds__(128) im2col_kernel(const T* __restrict__ x, T*
       }
     }
     __syncwarp();
-    const int n = (int)(ldc - k0 < 64 ? ldc - k0 : 64);
+    const int n = (int)(ldc - k0 < KT ? ldc - k0 : KT);
     if (vec) {
-      constexpr int kLanes = 64 / V;            // lanes per row
+      constexpr int kLanes = KT / V;            // lanes per row
       for (int i = lane; i < 32 * kLanes; i += 32) {
         const int rr = i / kLanes, cc = (i % kLanes) * V;
         if (r0 + rr < rows && cc < n)
           *reinterpret_cast<uint4*>(cols + (r0 + rr) * ldc + k0 + cc) = *reinterpret_cast<const uint4*>(st + rr * kPitch + cc);
       }
     } else {
-      for (int i = lane; i < 32 * 64; i += 32) {
-        const int rr = i >> 6, cc = i & 63;
+      for (int i = lane; i < 32 * KT; i += 32) {
+        const int rr = i / KT, cc = i % KT;
         if (r0 + rr < rows && cc < n) cols[(r0 + rr) * ldc + k0 + cc] = st[rr * kPitch + cc];
       }
     }
@@ -870,14 +888,28 @@ using namespace mmj;
 MMJ_API int mmj_im2col(const void* x, void* cols, const int* geom, long long ldc, int dtype, void* stream) {
   const ConvGeom g = make_geom(geom);
   if (!geom_ok(g) || ldc < (long long)g.C * g.kH * g.kW || ldc > 0x7fffffc0LL) return -2;
-  const long long units = ((long long)g.N * g.OH * g.OW + 31) / 32 * ((ldc + 63) / 64);
-  const long long blocks = (units + 3) / 4;
+  const long long total = (long long)g.N * g.OH * g.OW * ldc;
+  if (total <= 131072) {
+    const unsigned small_grid = (unsigned)((total + 255) / 256);
+    DISPATCH(dtype, (im2col_small_kernel<float><<<small_grid, 256, 0, STREAM>>>((const float*)x, (float*)cols, g, (int)ldc)),
+             (im2col_small_kernel<__nv_bfloat16><<<small_grid, 256, 0, STREAM>>>((const __nv_bfloat16*)x,
+                                                                                 (__nv_bfloat16*)cols, g, (int)ldc)));
+    return (int)cudaGetLastError();
+  }
+  const long long pos_tiles = ((long long)g.N * g.OH * g.OW + 31) / 32;
+  // 16 columns to a warp while 64 would leave an SM fewer than eight warps (times above the kernel)
+  const bool narrow = pos_tiles * ((ldc + 63) / 64) < 148 * 8;
+  const long long blocks = (pos_tiles * (narrow ? (ldc + 15) / 16 : (ldc + 63) / 64) + 3) / 4;
   const unsigned grid = (unsigned)(blocks < 148 * 32 ? blocks : 148 * 32);
   // 16-byte stores need rows that are whole vectors
   const int vec = ldc % (dtype == 1 ? 4 : 8) == 0 && ((uintptr_t)cols & 15) == 0;
-  DISPATCH(dtype, (im2col_kernel<float><<<grid, 128, 0, STREAM>>>((const float*)x, (float*)cols, g, ldc, vec)),
-           (im2col_kernel<__nv_bfloat16><<<grid, 128, 0, STREAM>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)cols, g, ldc,
-                                                                   vec)));
+  const float* xf = (const float*)x;
+  const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
+  if (dtype == 1 && narrow) im2col_kernel<float, 16><<<grid, 128, 0, STREAM>>>(xf, (float*)cols, g, ldc, vec);
+  else if (dtype == 1) im2col_kernel<float, 64><<<grid, 128, 0, STREAM>>>(xf, (float*)cols, g, ldc, vec);
+  else if (dtype == 0 && narrow) im2col_kernel<__nv_bfloat16, 16><<<grid, 128, 0, STREAM>>>(xb, (__nv_bfloat16*)cols, g, ldc, vec);
+  else if (dtype == 0) im2col_kernel<__nv_bfloat16, 64><<<grid, 128, 0, STREAM>>>(xb, (__nv_bfloat16*)cols, g, ldc, vec);
+  else return -1;
   return (int)cudaGetLastError();
 }
 MMJ_API int mmj_col2im(const void* cols, void* dx, const int* geom, long long ldc, int dtype, void* stream) {
