@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(256) sqnorm_partial_kernel(const T* __restrict
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
   // elements in front of the first 16-byte boundary and behind the last one are taken one by one
   long long head = (long long)((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) / (long long)sizeof(T);
-  if (head > n) head = n;
+  if (head > n || n <= step) head = n;
   const long long nv = (n - head) / V, tail = head + nv * V;
   const uint4* xv = reinterpret_cast<const uint4*>(x + head);
   for (long long i = tid; i < nv; i += 4 * step) {
@@ -500,13 +500,16 @@ MMJ_API int mmj_sgd(const void* g, int grad_dtype, float* w, float* mom, void* p
 MMJ_API int mmj_sqnorm_parts() { return 148 * 8; }
 MMJ_API int mmj_sqnorm(const void* x, int dtype, long long n, float* scratch, float* out,
                        int* found_inf, int accumulate, void* stream) {
-  const int parts = mmj_sqnorm_parts();
+  // No more blocks than have work: 1000 bf16 values took 5.0 us with all 1184, 3.3 now. Up to 592 blocks a thread takes
+  // one value, without the vector loop in front (100001 values: 3.8 us, 4.8 with it).
+  const long long round = n <= 592 * 256 ? 256 : 256 * 4 * (dtype == 0 ? 8 : 4), blocks = (n + round - 1) / round;
+  const int parts = blocks < 1 ? 1 : blocks < mmj_sqnorm_parts() ? (int)blocks : mmj_sqnorm_parts();
   if (dtype == 0)
     sqnorm_partial_kernel<__nv_bfloat16><<<parts, 256, 0, STREAM>>>((const __nv_bfloat16*)x, n,
                                                                    scratch, found_inf);
   else
     sqnorm_partial_kernel<float><<<parts, 256, 0, STREAM>>>((const float*)x, n, scratch, found_inf);
-  sqnorm_finalize_kernel<<<1, 256, 0, STREAM>>>(scratch, parts, out, accumulate);
+  sqnorm_finalize_kernel<<<1, parts > 256 ? 1024 : 256, 0, STREAM>>>(scratch, parts, out, accumulate);
   return (int)cudaGetLastError();
 }
 
