@@ -1233,9 +1233,20 @@ __device__ __forceinline__ void epilogue_cols8(const GemmParams& p, float (&v)[8
   }
   if (epi & kEpiOutF32) {
     float* d = reinterpret_cast<float*>(p.D) + (long long)row * p.ldd + col0;
+    if (full) {
+      float4* d4 = reinterpret_cast<float4*>(d);
+      if (epi & kEpiAccumulate) {
+        const float4 a = d4[0], b = d4[1];
+        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+        v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+      }
+      d4[0] = make_float4(v[0], v[1], v[2], v[3]);
+      d4[1] = make_float4(v[4], v[5], v[6], v[7]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (col0 + i < p.N) d[i] = (epi & kEpiAccumulate) ? d[i] + v[i] : v[i];
+      for (int i = 0; i < 8; ++i)
+        if (col0 + i < p.N) d[i] = (epi & kEpiAccumulate) ? d[i] + v[i] : v[i];
+    }
   } else {
     __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + (long long)row * p.ldd + col0;
     if (epi & kEpiAccumulate) {
