@@ -44,19 +44,25 @@ def _gelu_tanh_grad(x):
     return 0.5 * (1 + t) + 0.5 * x * (1 - t * t) * k0 * (1 + 3 * k1 * x * x)
 
 
-def pick_split(M: int, N: int, K: int) -> int:
-    """Ranges of K (1, 2, 4 or 8) for the split kernel, 0 where the larger tiles are the better ones. Measured, larger
-    tiles / split, us: 8 x 2304 x 768 9.8 / 8.3 (2 ranges; 4 ranges, 144 CTAs, 12.8: clusters of four no longer fit one
-    round), 113 x 768 x 3072 26.5 / 10.7 (8), 1 x 4096 x 4096 33.9 / 16.5 (2), 700 x 640 x 2000 14.4 / 11.6 (2),
-    64 x 8192 x 4096 34.4 / 25.0 (1). With more tiles than that a second range finds no SM and pairs of CTAs win
-    (1024 x 768 x 768 8.6 / 9.5), with a short contraction there is nothing to cut (64 x 64 x 64 4.3 / 5.9)."""
+def pick_split(M: int, N: int, K: int, heavy: bool = False) -> int:
+    """Ranges of K (1, 2, 4 or 8) for the split kernel, 0 where the larger tiles are the better ones. A range costs the
+    time of its K blocks (1.1 us for four) over a base that grows with the cluster and with the clusters that do not fit
+    one round. Measured, us, larger tiles / 1 / 2 / 4 / 8 ranges: 1 to 12 tiles, K = 768 9.1 / 8.4 / 7.0 / 7.5 / 8.6,
+    1536 14.6 / 11.7 / 8.7 / 8.3 / 9.0, 4096 32.8 / 22.6 / 14.3 / 11.1 / 10.2, 16 tiles, K = 4096 33.1 / 22.7 / 14.4 / 11.3 /
+    13.8 and 50304 365 / - / - / 65 / 47, 64 tiles, K = 4096 33.4 / 23.5 / 15.3 / 17.2 / 35.2. The CTAs of a cluster share
+    the epilogue, so that one with GELU or its derivative (``heavy``) pays for four earlier (16 x 768 x 768 two ranges 8.8,
+    four 7.6). One range pays from 64 rows on (9472 columns: 20 rows of K = 2048 18.9 / 21.7, 64 18.8 / 16.1) and 12 K
+    blocks (64 x 9472 x 512 7.7 / 8.6). Products of 256 rows and columns with more tiles go to pairs of CTAs."""
     tiles, blocks = -(-M // 128) * -(-N // 64), -(-K // 64)
     if blocks < 8 or tiles > (148 if M < 256 else 64) or (_PAIR["mode"] == "1" and M >= 256 and N >= 256):
         return 0     # (mode 1: the pair kernel wherever it can run)
-    s = 1
-    while s < 8 and tiles * s * 2 <= 128 and blocks >= 4 * s:
-        s *= 2
-    return s
+    if tiles > 64:
+        return 1 if M >= 64 and blocks >= 12 else 0
+    if tiles > 32:
+        return 2 if blocks < 112 else 4
+    if blocks < (8 if heavy else 24):
+        return 2
+    return 8 if blocks >= (48 if tiles <= 8 else 64 if tiles <= 12 else 128 if tiles <= 16 else 192) else 4
 
 
 def pick_bn(M: int, N: int) -> int:
@@ -294,7 +300,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_f32=False, accumulate=Fa
         if S > 1:
             return _gemm_split_k(a, b, out, accumulate, M, N, K, S, sbn, stall)
     if bn is None and not tall and pair is None and not a_mn:
-        s = pick_split(M, N, K)
+        s = pick_split(M, N, K, gelu or silu or dgelu_aux is not None)
         if s:
             bn, pair = SPLIT | s << 16, False
     if pair is None:

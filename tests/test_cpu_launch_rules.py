@@ -77,7 +77,8 @@ def test_split_rule_leaves_no_range_empty():
     for m in (1, 100, 128, 129, 255, 256, 700):
         for n in (8, 64, 72, 520, 2304):
             for k in (8, 64, 448, 512, 520, 576, 1024, 4096):
-                assert gemm_mod.pick_split(m, n, k) <= -(-k // 64)
+                for heavy in (False, True):
+                    assert gemm_mod.pick_split(m, n, k, heavy) <= -(-k // 64)
 
 
 def test_pair_mode_one_takes_every_eligible_product(monkeypatch):
@@ -119,3 +120,13 @@ def test_small_weight_gradients_stay_direct(n, c, hw, oc, k, direct):
 def test_bf16_input_gradient_takes_the_faster_route(n, c, hw, oc, k, stride, direct):
     o = (hw + 2 * (k // 2) - k) // stride + 1
     assert conv._direct_dx(n, c, hw, hw, oc, o, o, k * k, stride * stride) == direct
+
+
+@pytest.mark.parametrize("m,n,k,heavy,ranges", [
+    (8, 2304, 768, False, 2), (113, 768, 3072, False, 4), (113, 768, 4096, False, 8), (113, 768, 768, False, 2),
+    (113, 768, 768, True, 4), (1, 4096, 4096, False, 2), (1, 4096, 8192, False, 4), (16, 1024, 50304, False, 8),
+    (700, 640, 2000, False, 2), (64, 8192, 4096, False, 1), (8, 8192, 4096, False, 0), (16, 9472, 1024, True, 0),
+    (64, 9472, 512, False, 0), (512, 512, 512, False, 2), (1, 1024, 1024, False, 2), (256, 256, 1536, False, 4)])
+def test_few_tile_rule(m, n, k, heavy, ranges):
+    """Ranges by tiles and K blocks; few rows of many columns and short contractions of one range keep the larger tiles."""
+    assert gemm_mod.pick_split(m, n, k, heavy) == ranges
