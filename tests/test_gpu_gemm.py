@@ -151,8 +151,9 @@ def test_gemm_split_k_weight_gradient(force, M, N):
 @pytest.mark.parametrize("M,N,K", [(1, 8, 512), (113, 776, 776), (129, 72, 1000), (200, 64, 4096), (64, 8192, 520)])
 @pytest.mark.parametrize("splits", [1, 2, 4, 8])
 def test_split_kernel_edges(M, N, K, splits):
-    """Ragged rows, columns and K ranges of every cluster size, each epilogue option, against a product in 64 bits:
-    the result's own rounding to bf16 is 2^-9, fp32 results differ by the order of K additions."""
+    """Ragged rows, columns and K ranges of every cluster size, against a product in 64 bits: the result's own rounding to
+    bf16 is 2^-9, fp32 results differ by the order of K additions. The other epilogues and the element-wise stores are in
+    the next test."""
     from momijo_b200.ops.gemm import SPLIT
 
     g = torch.Generator(device="cuda").manual_seed(1)
@@ -176,11 +177,81 @@ def test_split_kernel_edges(M, N, K, splits):
     assert torch.equal(gemm(a, b, bn=bn), gemm(a, b, bn=bn))
 
 
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("M,N,K", [(113, 776, 776), (5, 500, 1000), (257, 61, 520)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_split_kernel_epilogues(M, N, K, splits, shift):
+    """Every epilogue of the split kernel by itself, with whole groups of eight columns and with partial ones, and with
+    operands that are not 16-byte aligned (shift), where it goes element by element. Results are rounded to bf16 (2^-9),
+    GELU' and SiLU add the 2^-11 of the hardware's tanh and exponential."""
+    from momijo_b200.ops.gemm import SPLIT
+
+    g = torch.Generator(device="cuda").manual_seed(8)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    ld = (N + 15) // 8 * 8
+    wide = lambda: r(M, ld)[:, shift:shift + N]           # a view of wider rows
+    a, b, bias, aux, bn = r(M, K), r(N, K) * K ** -0.5, r(N + 1)[shift:shift + N], wide(), SPLIT | splits << 16
+    rs = torch.rand(M, generator=g, device="cuda")
+    ref, x = a.double() @ b.double().t(), aux.double()
+
+    def close(want, tol=2.0 ** -8, **kw):
+        out = kw.pop("out", None)
+        out = torch.zeros(M, ld, device="cuda", dtype=torch.bfloat16)[:, :N] if out is None else out
+        assert gemm(a, b, bn=bn, out=out, **kw) is out
+        assert float((out.double() - want).norm()) <= tol * float(want.norm())
+
+    close(ref + bias.double(), bias=bias)
+    close(ref * _gelu_tanh_grad(x), dgelu_aux=aux)
+    close(ref * x, mul_aux=aux)
+    close(ref + x, add_aux=aux)
+    close(torch.nn.functional.silu(ref), silu=True)
+    close(ref * rs.double()[:, None], row_scale=rs)
+    acc = wide()
+    close(ref + acc.double(), out=acc, accumulate=True)
+    base = torch.randn(M, ld, generator=g, device="cuda")[:, shift:shift + N]
+    close(ref + base.double(), 4 * 2.0 ** -24 * K ** 0.5, out=base, accumulate=True)
+    close(ref, 4 * 2.0 ** -24 * K ** 0.5, out=torch.zeros(M, ld, device="cuda")[:, shift:shift + N])
+    pre, act = wide(), wide()
+    gemm(a, b, bn=bn, out=act, bias=bias, gelu=True, pre_out=pre)
+    for got, want in ((pre, ref + bias.double()), (act, _gelu_tanh(ref + bias.double()))):
+        assert float((got.double() - want).norm()) <= 2.0 ** -8 * float(want.norm())
+
+
+@pytest.mark.parametrize("M,N,K,fused", [
+    (768, 768, 16384, True), (2304, 768, 8192, True),
+    (320, 776, 9000, True),          # the last tile of rows and of columns and the last K block partly filled
+    (704, 2304, 16384, True),        # more tiles than pairs of CTAs: warps go on to a second one
+    (320, 520, 4100, False), (64, 64, 4096, False), (768, 768, 104, False)])
+@pytest.mark.parametrize("db_dtype,acc", [(torch.bfloat16, False), (torch.float32, True)])
+def test_bias_sums_from_the_stages(M, N, K, fused, db_dtype, acc):
+    """The fused form runs where the plan is a split one on CTA pairs, and nowhere else; column sums in fp32."""
+    from momijo_b200.ops.gemm import wgrad_bias
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    dy, x = r(K, M), r(K, N)
+    dw, db = r(M, N), r(M).to(db_dtype)
+    want_w = dy.double().t() @ x.double() + (dw.double() if acc else 0)
+    want_b = dy.double().sum(0) + (db.double() if acc else 0)
+    before = dw.clone(), db.clone()
+    assert wgrad_bias(dy, x, dw, acc, db, acc) == fused
+    if not fused:
+        assert torch.equal(dw, before[0]) and torch.equal(db, before[1])
+        return
+    assert float((dw.double() - want_w).norm()) <= 2.0 ** -8 * float(want_w.norm())
+    # sums of K values in chains of at most 128 (16 rows of 8 stages) and as many of those: well within 4 sqrt(K) 2^-24
+    tol = 2.0 ** -8 if db_dtype == torch.bfloat16 else 4 * 2.0 ** -24 * K ** 0.5
+    assert ((db.double() - want_b).abs() <= tol * want_b.abs() + 4 * 2.0 ** -24 * K ** 0.5 * K ** 0.5).all()
+    again = before[1].clone()
+    wgrad_bias(dy, x, before[0], acc, again, acc)
+    assert torch.equal(again, db)
+
+
 @pytest.mark.parametrize("M,N,K", [(768, 768, 16384), (320, 520, 4100), (2304, 768, 8192), (64, 64, 4096), (768, 768, 100)])
 @pytest.mark.parametrize("db_dtype,acc", [(torch.bfloat16, False), (torch.float32, True)])
 def test_weight_and_bias_gradient_together(M, N, K, db_dtype, acc):
-    """Column sums taken from the stages of a split weight gradient (tails of the last tile and of K among the shapes)
-    and from the separate pass where it is not split."""
+    """Both gradients of a linear layer into gradient buffers: from one product where the plan is a split one, from a
+    product and a separate pass elsewhere (test_bias_sums_from_the_stages says which is which)."""
     from momijo_b200.ops import functional as fn
 
     g = torch.Generator(device="cuda").manual_seed(2)
