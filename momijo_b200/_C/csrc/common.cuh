@@ -343,14 +343,8 @@ __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc
       : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on one mbarrier (either CTA of the pair) once the pair MMAs issued so far have completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar_cluster_addr)
-               : "memory");
-}
-
-// The same arrival on the mbarrier at one shared-memory offset in both CTAs of the pair, in one instruction.
+// Arrive on the mbarrier at one shared-memory offset in both CTAs of the pair, in one instruction, once the pair MMAs
+// issued so far have completed.
 __device__ __forceinline__ void umma_commit_pair_both(uint64_t* bar) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
