@@ -2,10 +2,11 @@
 // GQA, head_dim 64 or 128), with Q/K/V/dO tiles staged by TMA (128-byte swizzle) and every
 // matrix product accumulated in tensor memory.
 //
-// Forward, one CTA per (128 query rows, head, batch):
+// Forward (attn_fwd3_kernel), per item of 256 query rows of one (head, batch), looping over blocks of 64 keys:
 //   S = Q K^T in TMEM -> softmax warps read one row per thread (no shuffles needed), keep the
-//   running max / sum, write P (bf16) into shared memory in the swizzled K-major layout ->
-//   O_part = P V in TMEM -> threads fold O_part into a register accumulator.
+//   running max / sum, write P (bf16) back over S in TMEM -> O += P V in TMEM, rescaled in place when
+//   the maximum has grown by much. attn_fwd_kernel is the older form: one CTA per 128 query rows, P
+//   through shared memory, O folded into registers.
 // Backward, per item of 128 key rows of one (kv head, batch), looping over the query blocks (and,
 // for GQA, over the query heads of the group):
 //   S^T = K Q^T and dP^T = V dO^T (TMEM) -> threads rebuild P^T = exp(S^T*scale - lse) and
@@ -409,9 +410,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 //     (S_t[0], S_t[1], 64 columns each): the MMA thread issues S_t(j+1) before the group has finished
 //     block j, so a group that has stored P_t(j) finds S_t(j+1) waiting and starts on it at once;
 //     per key block the MMA thread does  [wait P_t(j)]  P_t(j) V_j -> O_t,  Q_t K_(j+2)^T -> S_t[j & 1];
-//   * the softmax is bound by issue (two warps per scheduler at 60 % of the slots): three-operand maxima, paired
-//     multiply-adds and sums and the paired conversion take 192 instructions for 64 scores where scalar ones and
-//     integer rounding took 352.
+//   * three-operand maxima, paired multiply-adds and sums and the paired conversion shorten the softmax's own chain
+//     (B6 T1777 H16 D128 full 196 -> 183 us).
+// No unit bounds it: counters of that call read issue slots 34 %, exponentials' unit 46 % (64 exponentials and 32
+// conversions a row and block), tensor pipe 45 %, L2 21 %; at head_dim 64 (B16 T1024 H12 causal) 34, 41, 20 and 15 %.
+// 0.46 warps are ready a cycle and scheduler, out of three: fixed-latency waits (2.3 of 8.8 cycles an instruction), TMEM
+// loads (1.4 and 1.8) and the stores' queue (1.0 and 0.5) are the chain of one row per thread, one warp a scheduler and tile.
 // Tensor memory: S0[0] S0[1] S1[0] S1[1] | O0 | O1 = 256 + 2 D columns; P_t(j) overwrites the first 32
 // columns of S_t[j & 1] (64 probabilities as bf16 pairs). Every P_t(j) V_j commits to o_done[t][j & 1];
 // a group waits on it only before it rescales O_t (rare: the running maximum must have grown by more
@@ -927,7 +931,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sKV = smem;                          // kKV x (K | V)
   uint8_t* sQO = sKV + kKV * 2 * kTile;         // kStages x (Q | dO)
-  uint8_t* sdS = sQO + kStages * 2 * kQTile;    // 2 x dS^T
+  uint8_t* sdS = sQO + kStages * 2 * kQTile;    // kBufs x dS^T
   uint8_t* sDQ = sdS + kBufs * kDsBytes;            // 4 warps x 2
   typedef BwdCtl<8 * kGroups> Ctl;
   Ctl& ctl = *reinterpret_cast<Ctl*>(sDQ + 8 * kDqBytes);

@@ -708,8 +708,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 constexpr int kPairBN = 256;
 constexpr int kPairStageBytes = kAStageBytes + (kPairBN / 2) * kGemmBK * 2;  // 32 KiB
 
-// The fused GELU / GELU' epilogues are bound by issue (25 and 28 instructions an element at 41 % of the issue slots with
-// scalar arithmetic, two or three warps per scheduler), not by a pipe.
+// The fused GELU / GELU' epilogues lengthen the chain of a tile's 32-column chunks; no unit bounds them. Counters at
+// 16384 x 3072 x 768, bias only / GELU / GELU': tensor pipe 72 / 52 / 50 %, issue slots 19 / 25 / 27 %, exponentials' unit 1 /
+// 18 / 17 %, 6 / 11 / 13 instructions an element, 2.5 warps a scheduler that mostly wait for TMEM and shared memory.
 // the two bf16 halves of a word, widened (their bits are the upper halves of the fp32 values)
 __device__ __forceinline__ f32x2 f2_from_bf16(uint32_t u) {
   return f2_pack(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
@@ -1172,11 +1173,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
 // Split kernel: 128 x 64 tiles whose contraction is cut over a cluster of S CTAs
 // ---------------------------------------------------------------------------------------------
 // For products with few output tiles (a handful of rows through a projection, short prompts). There the time is one
-// CTA's walk along K, about 1000 cycles for each 64-deep block (one SM's share of the L2 plus latency), while most SMs
-// idle: 8 x 2304 x 768 took 14.1 us on 18 CTAs, 113 x 768 x 3072 40 us on 6. Narrow tiles and up to eight ranges of K
-// put the operands' bytes on as many SMs as there are; the partial tiles meet in distributed shared memory, where CTA r
-// of a cluster adds columns [64 r / S, 64 (r + 1) / S) over the ranks in order (the result does not depend on timing)
-// and runs the epilogue on them: 8.3 us and 10.6 us (2 and 8 ranges of K; the rule that picks them is the front end's).
+// CTA's walk along K, about 900 cycles for each 64-deep block (one SM's share of the L2 plus latency), while most SMs
+// idle: 16 x 2304 x 768 takes 9.4 us on 18 CTAs, 113 x 768 x 3072 26.0 us on 6. Narrow tiles (500 cycles a block) and up
+// to eight ranges of K put the operands' bytes on as many SMs as there are; the partial tiles meet in distributed shared
+// memory, where CTA r of a cluster adds columns [64 r / S, 64 (r + 1) / S) over the ranks in order (the result does not
+// depend on timing) and runs the epilogue on them: 7.3 us and 10.3 us (2 and 4 ranges of K; the rule that picks them, with
+// every count's time, is the front end's).
 constexpr int kSplitBN = 64, kSplitStages = 4, kSplitThreads = 192;
 constexpr int kSplitStageBytes = kAStageBytes + kSplitBN * kGemmBK * 2;   // 24 KiB
 constexpr int kSplitPitch = 68;                                          // floats; rows 16-byte aligned, conflict free

@@ -51,8 +51,8 @@ def pick_split(M: int, N: int, K: int, heavy: bool = False) -> int:
     1536 14.6 / 11.7 / 8.7 / 8.3 / 9.0, 4096 32.8 / 22.6 / 14.3 / 11.1 / 10.2, 16 tiles, K = 4096 33.1 / 22.7 / 14.4 / 11.3 /
     13.8 and 50304 365 / - / - / 65 / 47, 64 tiles, K = 4096 33.4 / 23.5 / 15.3 / 17.2 / 35.2. The CTAs of a cluster share
     the epilogue, so that one with GELU or its derivative (``heavy``) pays for four earlier (16 x 768 x 768 two ranges 8.8,
-    four 7.6). One range pays from 64 rows on (9472 columns: 20 rows of K = 2048 18.9 / 21.7, 64 18.8 / 16.1) and 12 K
-    blocks (64 x 9472 x 512 7.7 / 8.6). Products of 256 rows and columns with more tiles go to pairs of CTAs."""
+    four 7.6). One range pays from 64 rows on (9472 columns: 20 rows of K = 2048 18.9 / 21.7, 64 19.0 / 15.4) and 12 K
+    blocks (64 x 9472 x 512 7.7 / 8.7). Products of 256 rows and columns with more tiles go to pairs of CTAs."""
     tiles, blocks = -(-M // 128) * -(-N // 64), -(-K // 64)
     if blocks < 8 or tiles > (148 if M < 256 else 64) or (_PAIR["mode"] == "1" and M >= 256 and N >= 256):
         return 0     # (mode 1: the pair kernel wherever it can run)
