@@ -840,10 +840,12 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ O, long long
 // of TMEM, 2 = issuer of the gradient products, 3 = idle, then one (head_dim 128) or two (64) compute groups of eight
 // warps, then four dQ drain warps.
 //
-// What bounds it: a block's chain - scores 1060 cycles, TMEM read / exponential / store 1430, gradients 1230, measured
-// with clock stamps at head_dim 64 - is twice as long as the tensor core's own time (about 55 cycles for each of 24 or 32
-// products, which read 2 to 4 KB of A and B from shared memory each), so blocks have to overlap; at head_dim 128 the
-// L2's rate of fp32 reductions costs another sixth (785 -> 655 us without them).
+// What bounds it: a block's chain, by the clock stamps at head_dim 64 (B16 T1024 H12): 240 cycles to read the scores, 1320
+// for the exponentials and the stores, 140 to the gradient issuer, 1980 until dQ^T is complete behind the products queued
+// before it. It is several times the tensor core's own time (about 55 cycles for each of 24 or 32 products, which read 2 to 4
+// KB of A and B from shared memory each), so blocks have to overlap: one every 1790 cycles, at 52 % of the issue slots, 35 %
+// of the tensor pipe and 39 % of the shared-memory pipe. At head_dim 128 (B2 T4096 H32:8: 190, 1120, 150, 790, one every 2390) the L2's
+// rate of fp32 reductions costs another sixth (785 -> 655 us without them).
 //   * 64 queries to a block, because two 128-query blocks do not fit (at head_dim 128 one block of 128 left a single
 //     Q / dO stage, and every block waited out a TMA round trip). Three blocks are in flight at head_dim 64, where two
 //     compute groups take them in turn (two blocks and one group: 160 us against 151; sixteen warps on one block: 170);
