@@ -178,16 +178,18 @@ __device__ __forceinline__ void rotate8(float (&a)[8], float (&b)[8], const floa
     a[j] = na; b[j] = nb;
   }
 }
+// (kOneRow: the row and its table entries stay out of the loop; 4096 rows of 32:8 heads of 128 16.7 us, 17.8 without)
+template <bool kOneRow>
 __global__ void __launch_bounds__(256) rope_copy_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst,
                                                         const float2* __restrict__ cs, long long ld, int n_rot,
                                                         int n_heads, int D, int T, int rows, int block_rows) {
   pdl_wait();
   pdl_trigger();
   const int half = D >> 1, per_head = half >> 3, per_row = n_heads * per_head;
-  for (int i = threadIdx.x; i < block_rows * per_row; i += blockDim.x) {
-    const int rr = block_rows == 1 ? 0 : i / per_row, w = i - rr * per_row;
-    const long long r = (long long)blockIdx.x * block_rows + rr;
-    if (r >= rows) break;
+  for (int i = threadIdx.x; i < (kOneRow ? per_row : block_rows * per_row); i += blockDim.x) {
+    const int rr = kOneRow ? 0 : i / per_row, w = i - rr * per_row;
+    const long long r = kOneRow ? (long long)blockIdx.x : (long long)blockIdx.x * block_rows + rr;
+    if (!kOneRow && r >= rows) break;
     const float2* t = cs + (size_t)((unsigned)r % (unsigned)T) * half;
     const int h = w / per_head, c = (w - h * per_head) * 8;
     const long long off = r * ld + h * D + c;
@@ -670,7 +672,7 @@ MMJ_API int mmj_rope_copy(const void* src, void* dst, const float* cos_sin, long
   if (D % 16 || ld % 8 || (((uintptr_t)src | (uintptr_t)dst) & 15) || rows > 0x7fffffffLL) return -1;
   if (rows == 0 || n_heads == 0) return 0;
   const int block_rows = rope_block_rows(rows, n_heads, D);
-  launch_pdl(rope_copy_kernel, dim3((unsigned)((rows + block_rows - 1) / block_rows)), dim3(256), 0, STREAM,
+  launch_pdl(block_rows == 1 ? &rope_copy_kernel<true> : &rope_copy_kernel<false>, dim3((unsigned)((rows + block_rows - 1) / block_rows)), dim3(256), 0, STREAM,
              (const __nv_bfloat16*)src, (__nv_bfloat16*)dst, (const float2*)cos_sin, ld, n_rot, n_heads, D, T, (int)rows,
              block_rows);
   return (int)cudaGetLastError();
