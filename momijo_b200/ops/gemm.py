@@ -162,7 +162,7 @@ def pick_pair(M: int, N: int, K: int) -> bool:
 
 
 def _split_ranges(K: int, S: int, device):
-    key = (K, S, str(device))
+    key = (K, S, device)
     r = _SPLITK["ranges"].get(key)
     if r is None:
         step = -(-K // S)
@@ -185,26 +185,27 @@ def wgrad_bias(dy, x, out, accumulate, db, db_accumulate) -> bool:
     if S <= 1 or tall != "pair":
         return False
     lddy, ldx = _check_2d(dy, "a"), _check_2d(x, "b")
-    # slabs of this call's own: calls on other streams or threads run between the product and its fold
-    sc = dy.new_empty(S * M * N, dtype=torch.float32)
-    part = dy.new_empty(S * M, dtype=torch.float32)
-    _C.call("mmj_wgrad_bias", dy.data_ptr(), lddy, x.data_ptr(), ldx, sc.data_ptr(), part.data_ptr(), K, M, N, S,
-            _C.ptr(_split_ranges(K, S, dy.device)), _C.status_tensor(dy.device).data_ptr(), _C.current_stream())
+    # slabs of this call's own, the bias sums behind them: calls on other streams or threads run between the product and
+    # its fold
+    sc = dy.new_empty(S * M * (N + 1), dtype=torch.float32)
+    slabs, dev, stream = sc.data_ptr(), dy.device, _C.current_stream()
+    part = slabs + 4 * S * M * N
+    _C.call("mmj_wgrad_bias", dy.data_ptr(), lddy, x.data_ptr(), ldx, slabs, part, K, M, N, S,
+            _split_ranges(K, S, dev).data_ptr(), _C.status_tensor(dev).data_ptr(), stream)
     f32 = db.dtype == torch.float32
-    _C.call("mmj_wgrad_fold", sc.data_ptr(), M * N, S, out.data_ptr(), M * N, int(accumulate), part.data_ptr(), M,
-            None if f32 else db.data_ptr(), db.data_ptr() if f32 else None, int(db_accumulate), _C.current_stream())
+    _C.call("mmj_wgrad_fold", slabs, M * N, S, out.data_ptr(), M * N, int(accumulate), part, M,
+            None if f32 else db.data_ptr(), db.data_ptr() if f32 else None, int(db_accumulate), stream)
     return True
 
 
 def _gemm_split_k(a, b, out, accumulate, M, N, K, S, bn, tall=False):
     """a: [K, M], b: [K, N] (both MN-major). Partial products as fp32 slabs, then one reduction pass."""
     sc = a.new_empty(S * M * N, dtype=torch.float32)   # of this call's own, as in wgrad_bias
-    _C.call("mmj_gemm_bf16_grouped_k", _C.ptr(a), a.stride(0), _C.ptr(b), b.stride(0), _C.ptr(sc), N, K, M, N, S,
-            _C.ptr(_split_ranges(K, S, a.device)), 1, 0,
-            bn | (PAIR if tall == "pair" else TALL if tall else 0),
-            _C.ptr(_C.status_tensor(a.device)),
-            _C.current_stream())
-    _C.call("mmj_splitk_reduce", _C.ptr(sc), M * N, S, _C.ptr(out), M * N, int(accumulate), _C.current_stream())
+    slabs, dev, stream = sc.data_ptr(), a.device, _C.current_stream()
+    _C.call("mmj_gemm_bf16_grouped_k", a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), slabs, N, K, M, N, S,
+            _split_ranges(K, S, dev).data_ptr(), 1, 0, bn | (PAIR if tall == "pair" else TALL if tall else 0),
+            _C.status_tensor(dev).data_ptr(), stream)
+    _C.call("mmj_splitk_reduce", slabs, M * N, S, out.data_ptr(), M * N, int(accumulate), stream)
     return out
 
 
