@@ -84,7 +84,9 @@ def _direct_dx(N, C, H, W, OC, OH, OW, taps, classes):
     14 and 18 %): the direct kernel by its chain of 16-deep chunks and its multiply-adds, padding of its tiles
     included, the product by the patch matrix, the sums' reads and dy. The margin leaves 0.5 % of the shapes more than
     5 % slower than with the product, by 1.18 at most. Direct / product, k3: N32 C64 56x56 16 filters 83 / 282, 32 143 / 290, N1 C512
-    14x14 48 filters 33 / 22; k5: N1 C32 14x14 48 filters 61 / 19; k11: N4 C1 224x224 32 filters 1039 / 156."""
+    14x14 48 filters 33 / 22; k5: N1 C32 14x14 48 filters 61 / 19; k11: N4 C1 224x224 32 filters 1039 / 156. Up to 35 us the
+    direct kernel is taken all the same: the product's route needs 28 us more of the host, and a backward call whose
+    kernels are that short waits for the host (N4 C48 20x20 48 filters, both gradients: 86 us direct, 113)."""
     P = N * -(-H * W // classes)
     bm = 16 if C <= 16 else 32 if 1 <= C % 64 <= 32 else 64         # as the launcher chooses it
     blocks = lambda rows: -(-P // 128) * -(-C // rows) * classes
@@ -93,7 +95,7 @@ def _direct_dx(N, C, H, W, OC, OH, OW, taps, classes):
     K = OC * taps / classes
     direct = 7.4 + 0.66 * K / 16 + 55e-9 * blocks(bm) * 128 * bm * K
     product = 14.0 + 1e-6 * (1.5 * N * OH * OW * C * taps + 2.3 * N * C * H * W * taps + 6.5 * N * OH * OW * OC)
-    return direct < 0.85 * product
+    return direct < 35 or direct < 0.85 * product
 
 
 def _weight_grad(x, dy, w, geom):

@@ -114,7 +114,8 @@ def test_small_weight_gradients_stay_direct(n, c, hw, oc, k, direct):
 
 @pytest.mark.parametrize("n,c,hw,oc,k,stride,direct", [
     (32, 64, 56, 16, 3, 1, True), (32, 64, 56, 32, 3, 1, True), (32, 64, 56, 64, 1, 1, True),
-    (1, 512, 14, 48, 3, 1, False), (2, 48, 20, 48, 3, 1, False), (1, 32, 14, 48, 5, 1, False),   # few positions
+    (1, 512, 14, 48, 3, 1, True), (4, 48, 20, 48, 3, 1, True),      # both short: the product's route waits for the host
+    (1, 32, 14, 48, 5, 1, False), (1, 64, 28, 96, 3, 1, False),                                 # few positions
     (4, 1, 224, 32, 11, 1, False), (16, 3, 56, 32, 5, 1, False),                                # rows of padding
     (32, 64, 56, 128, 3, 1, False)])
 def test_bf16_input_gradient_takes_the_faster_route(n, c, hw, oc, k, stride, direct):
