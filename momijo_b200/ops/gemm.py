@@ -179,7 +179,7 @@ def wgrad_bias(dy, x, out, accumulate, db, db_accumulate) -> bool:
     K, M = dy.shape
     N = x.shape[1]
     if (not dy.is_cuda or out.dtype != torch.bfloat16 or not out.is_contiguous() or not db.is_contiguous()
-            or M % 64 or N % 8):
+            or M % 64 or N % 8 or out.data_ptr() % 16):      # the fold stores 16 bytes at a time
         return False
     S, _, tall = plan_wgrad(M, N, K)
     if S <= 1 or tall != "pair":
@@ -296,7 +296,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_f32=False, accumulate=Fa
     if N % 8 != 0 and ldo % 8 != 0:
         raise ValueError("output leading dimension must be a multiple of 8 elements")
     if (a_mn and b_mn and epi in (0, EPI_ACCUMULATE) and out.is_contiguous() and (M * N) % 8 == 0
-            and M % 8 == 0 and N % 8 == 0):
+            and M % 8 == 0 and N % 8 == 0 and out.data_ptr() % 16 == 0):
         S, sbn, stall = plan_wgrad(M, N, K)
         if S > 1:
             return _gemm_split_k(a, b, out, accumulate, M, N, K, S, sbn, stall)

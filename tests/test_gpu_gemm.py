@@ -247,6 +247,20 @@ def test_bias_sums_from_the_stages(M, N, K, fused, db_dtype, acc):
     assert torch.equal(again, db)
 
 
+def test_weight_gradient_into_a_misaligned_buffer():
+    """A contiguous buffer that does not start on 16 bytes takes the plain product, whose epilogue stores by elements."""
+    from momijo_b200.ops.gemm import wgrad_bias
+
+    g = torch.Generator(device="cuda").manual_seed(9)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    dy, x = r(8192, 768), r(8192, 768)
+    out = torch.zeros(768 * 768 + 1, device="cuda", dtype=torch.bfloat16)[1:].view(768, 768)
+    assert not wgrad_bias(dy, x, out, False, r(768), False) and not out.any()
+    gemm(dy, x, a_mn=True, b_mn=True, out=out)
+    want = dy.double().t() @ x.double()
+    assert float((out.double() - want).norm()) <= 2.0 ** -8 * float(want.norm())
+
+
 @pytest.mark.parametrize("M,N,K", [(768, 768, 16384), (320, 520, 4100), (2304, 768, 8192), (64, 64, 4096), (768, 768, 100)])
 @pytest.mark.parametrize("db_dtype,acc", [(torch.bfloat16, False), (torch.float32, True)])
 def test_weight_and_bias_gradient_together(M, N, K, db_dtype, acc):
