@@ -621,9 +621,14 @@ static inline int grid_for(long long work, int threads) {
 using namespace mmj;
 #define STREAM ((cudaStream_t)stream)
 
+// Kernels that move 16 bytes at a time: a view at an odd offset is refused here (-3), not found out by a fault.
+static inline bool off16(const void* a, const void* b = nullptr, const void* c = nullptr) {
+  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) != 0;
+}
 MMJ_API int mmj_act_fwd(const void* x, void* y, long long n, int op, float alpha, void* stream) {
   if (n % 8) return -1;
   if (n == 0) return 0;
+  if (off16(x, y)) return -3;
   launch_pdl(act_fwd_kernel, dim3(grid_for(n / 8, 256)), dim3(256), 0, STREAM, (const __nv_bfloat16*)x,
              (__nv_bfloat16*)y, n / 8, op, alpha);
   return (int)cudaGetLastError();
@@ -632,6 +637,7 @@ MMJ_API int mmj_act_bwd(const void* x, const void* dy, void* dx, long long n, in
                         void* stream) {
   if (n % 8) return -1;
   if (n == 0) return 0;
+  if (off16(x, dy, dx)) return -3;
   launch_pdl(act_bwd_kernel, dim3(grid_for(n / 8, 256)), dim3(256), 0, STREAM, (const __nv_bfloat16*)x,
              (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, n / 8, op, alpha);
   return (int)cudaGetLastError();
@@ -639,6 +645,7 @@ MMJ_API int mmj_act_bwd(const void* x, const void* dy, void* dx, long long n, in
 MMJ_API int mmj_swiglu_fwd(const void* gu, void* y, long long rows, int F, void* stream) {
   if (F % 8) return -1;
   if (rows == 0) return 0;
+  if (off16(gu, y)) return -3;
   launch_pdl(swiglu_fwd_kernel, dim3(grid_for(rows * (F / 8), 256)), dim3(256), 0, STREAM,
              (const __nv_bfloat16*)gu, (__nv_bfloat16*)y, rows, F);
   return (int)cudaGetLastError();
@@ -647,6 +654,7 @@ MMJ_API int mmj_swiglu_bwd(const void* gu, const void* dy, void* dgu, long long 
                            void* stream) {
   if (F % 8) return -1;
   if (rows == 0) return 0;
+  if (off16(gu, dy, dgu)) return -3;
   launch_pdl(swiglu_bwd_kernel, dim3(grid_for(rows * (F / 8), 256)), dim3(256), 0, STREAM,
              (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dgu, rows, F);
   return (int)cudaGetLastError();
@@ -655,6 +663,7 @@ MMJ_API int mmj_rope(void* x, const void* cos_sin, long long rows, long long ld,
                      int n_heads, int D, int T, float sign, void* stream) {
   if (D % 16 || ld % 8 || head_off % 8) return -1;
   if (rows == 0 || n_heads == 0) return 0;
+  if (off16(x)) return -3;
   const long long work = rows * n_heads * (D / 16);
   launch_pdl(rope_kernel, dim3(grid_for(work, 256)), dim3(256), 0, STREAM, (__nv_bfloat16*)x,
              (const float2*)cos_sin, rows, ld, head_off, n_heads, D, T, sign);
@@ -691,6 +700,7 @@ MMJ_API int mmj_embedding_fwd(const long long* tok, const void* wte, const void*
                               long long rows, int C, int T, int vocab, void* stream) {
   if (C % 8) return -1;
   if (rows == 0) return 0;
+  if (off16(wte, wpe, out)) return -3;
   embedding_fwd_kernel<<<grid_for(rows * (C / 8), 256), 256, 0, STREAM>>>(
       tok, (const __nv_bfloat16*)wte, (const __nv_bfloat16*)wpe, (__nv_bfloat16*)out, rows, C, T,
       vocab);
@@ -701,6 +711,7 @@ MMJ_API int mmj_embedding_bwd(const long long* tok, const void* dout, void* dwte
                               void* stream) {
   if (C % 8) return -1;
   if (rows == 0) return 0;
+  if (((uintptr_t)dout | (uintptr_t)dwte) & 3 || (dwpe != nullptr && off16(dout, dwpe))) return -3;
   if (dwte != nullptr)
     embedding_bwd_wte_kernel<<<grid_for(rows * (C / 2), 256), 256, 0, STREAM>>>(
         tok, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dwte, rows, C, vocab);
@@ -721,6 +732,7 @@ MMJ_API int mmj_colsum_bf16(const void* x, long long ldx, void* out_bf16, float*
                             float* scratch, int M, int N, int accumulate, void* stream) {
   if (M <= 0 || N <= 0) return 0;
   if (ldx % 8) return -1;
+  if (off16(x)) return -3;
   const int S = mmj_colsum_splits(M);
   dim3 grid((N + 63) / 64, S);
   launch_pdl(colsum_partial_kernel, grid, dim3(256), 0, STREAM, (const __nv_bfloat16*)x, ldx, scratch, M, N);
@@ -734,6 +746,7 @@ MMJ_API int mmj_splitk_reduce(const float* parts, long long slab, int S, void* o
                               int accumulate, void* stream) {
   if (n == 0) return 0;
   if (n % 8 || slab % 4 || S < 1) return -1;
+  if (off16(parts, out)) return -3;
   launch_pdl(splitk_reduce_kernel, dim3(grid_for(n / 8, 256)), dim3(256), 0, STREAM, parts, slab, S,
              (__nv_bfloat16*)out, n, accumulate, (const float*)nullptr, 0, (__nv_bfloat16*)nullptr, (float*)nullptr, 0);
   return (int)cudaGetLastError();
@@ -743,6 +756,7 @@ MMJ_API int mmj_wgrad_fold(const float* parts, long long slab, int S, void* out,
                            const float* bias_part, int M, void* db, float* db32, int db_accumulate, void* stream) {
   if (n % 8) return -1;
   if (n == 0) return 0;
+  if (off16(parts, out)) return -3;
   launch_pdl(splitk_reduce_kernel, dim3(grid_for(n / 8, 256)), dim3(256), 0, STREAM, parts, slab, S,
              (__nv_bfloat16*)out, n, accumulate, bias_part, M, (__nv_bfloat16*)db, db32, db_accumulate);
   return (int)cudaGetLastError();

@@ -782,6 +782,8 @@ MMJ_API int mmj_norm_fwd(const void* x, const void* res, void* res_out, const vo
       if (launched) return (int)cudaGetLastError();
     }
   }
+  // the row kernels move 16 bytes at a time as well
+  if (!aligned16(x) || !aligned16(res) || !aligned16(y) || !aligned16(res_out) || !aligned16(gamma) || !aligned16(beta)) return -3;
   const int vpt = (C / 8 > 512) ? 2 : 1;  // at most 512 threads: the row kernels need over 64 registers
   const int threads = norm_threads(C, vpt);
   const int grid = rows;
@@ -848,6 +850,7 @@ MMJ_API int mmj_norm_bwd(const void* dy, const void* x, const void* gamma, const
       }
     }
   }
+  if (!aligned16(x) || !aligned16(dy) || !aligned16(dx) || !aligned16(dres_in) || !aligned16(gamma)) return -3;
   const int vpt = (C / 8 > 512) ? 2 : 1;  // at most 512 threads: the row kernels need over 64 registers
   const int threads = norm_threads(C, vpt);
   const bool prefetch = threads <= 256;

@@ -131,3 +131,21 @@ def test_bf16_input_gradient_takes_the_faster_route(n, c, hw, oc, k, stride, dir
 def test_few_tile_rule(m, n, k, heavy, ranges):
     """Ranges by tiles and K blocks; few rows of many columns and short contractions of one range keep the larger tiles."""
     assert gemm_mod.pick_split(m, n, k, heavy) == ranges
+
+
+@pytest.mark.parametrize("name,args", [
+    ("mmj_norm_fwd", (2, 0, 0, 16, 16, 16, None, 16, 4, 64, 1e-5, 1, None, None)),
+    ("mmj_norm_fwd", (16, 0, 0, 18, 16, 16, None, 16, 4, 64, 1e-5, 1, None, None)),
+    ("mmj_norm_bwd", (18, 16, 16, None, 16, None, 16, 16, None, 16, 4, 64, 1, 0, None, None)),
+    ("mmj_act_fwd", (18, 16, 64, 0, 0.0, None)), ("mmj_act_bwd", (16, 20, 16, 64, 0, 0.0, None)),
+    ("mmj_swiglu_fwd", (18, 16, 4, 16, None)), ("mmj_swiglu_bwd", (16, 16, 24, 4, 16, None)),
+    ("mmj_rope", (18, 16, 4, 64, 0, 1, 64, 4, 1.0, None)),
+    ("mmj_embedding_fwd", (16, 18, None, 16, 4, 64, 4, 10, None)),
+    ("mmj_embedding_bwd", (16, 18, 16, None, 4, 64, 4, 10, 0, None)),
+    ("mmj_embedding_bwd", (16, 20, 16, 16, 4, 64, 4, 10, 0, None)),
+    ("mmj_colsum_bf16", (18, 64, 16, None, 16, 4, 64, 0, None)),
+    ("mmj_splitk_reduce", (16, 64, 2, 18, 64, 0, None)),
+    ("mmj_wgrad_fold", (16, 64, 2, 18, 64, 0, 16, 8, 16, None, 0, None))])
+def test_vector_kernels_refuse_misaligned_operands(name, args):
+    """Views at odd offsets are refused on the host, before a launch (the addresses here are never read)."""
+    assert getattr(_C.lib(), name)(*args) == -3
