@@ -247,6 +247,35 @@ def test_bias_sums_from_the_stages(M, N, K, fused, db_dtype, acc):
     assert torch.equal(again, db)
 
 
+def test_split_weight_gradients_on_two_streams():
+    """Split weight gradients of different sizes side by side, with and without the bias sums, give the bits that each
+    gives alone (their slabs are their own)."""
+    from momijo_b200.ops.gemm import wgrad_bias
+
+    g = torch.Generator(device="cuda").manual_seed(10)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    jobs = []
+    for m, n, k, fused in ((768, 768, 16384, True), (2304, 768, 8192, True), (320, 520, 4104, False), (768, 3072, 8192, False)):
+        jobs.append((r(k, m), r(k, n), fused))
+
+    def run(dy, x, fused):
+        dw, db = torch.empty(dy.shape[1], x.shape[1], device="cuda", dtype=torch.bfloat16), dy.new_empty(dy.shape[1])
+        if fused:
+            assert wgrad_bias(dy, x, dw, False, db, False)
+            return dw, db
+        return (gemm(dy, x, a_mn=True, b_mn=True, out=dw),)
+
+    alone = [run(*j) for j in jobs]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream(), torch.cuda.Stream()], []
+    for i in range(12):
+        with torch.cuda.stream(streams[i % 2]):
+            got.append((i * 5 % 4, run(*jobs[i * 5 % 4])))
+    torch.cuda.synchronize()
+    for j, out in got:
+        assert all(torch.equal(a, b) for a, b in zip(out, alone[j]))
+
+
 def test_weight_gradient_into_a_misaligned_buffer():
     """A contiguous buffer that does not start on 16 bytes takes the plain product, whose epilogue stores by elements."""
     from momijo_b200.ops.gemm import wgrad_bias
